@@ -30,7 +30,7 @@ from uniserve_v1_b200.models.zonopel import ZonopelConfig, ZonopelModel
 
 BF16, F32, F64 = torch.bfloat16, torch.float32, torch.float64
 VOCAB, PAGE = 32000, 16
-ROUTER = 4.0            # gain of the routers' logits
+ROUTER, DOWN = 6.0, 0.5  # gain of the routers' logits, and of what a routed expert adds to the stream
 LAYERED = {"nepevik": (NepevikConfig, NepevikModel), "zonopel": (ZonopelConfig, ZonopelModel),
            "tadinex": (TadinexConfig, TadinexModel), "nopuzen": (NopuzenConfig, NopuzenModel)}
 CHUNK = 8192            # rows that an engine hands over at a time (``max_num_batched_tokens`` of the benchmark)
@@ -191,7 +191,7 @@ def _qwen_weights(d, c):
         d.around(p + "self_attn.k_norm.weight", D)
         d.lin(p + "mlp.gate.weight", E, H, gain=ROUTER)
         d.lin(p + "mlp.experts.gate_up_proj", E, 2 * I, H)
-        d.lin(p + "mlp.experts.down_proj", E, H, I)
+        d.lin(p + "mlp.experts.down_proj", E, H, I, gain=DOWN)
 
 
 def _hybrid_weights(d, c):
@@ -226,7 +226,7 @@ def _hybrid_weights(d, c):
         m = p + "mlp."
         d.lin(m + "gate.weight", E, H, gain=ROUTER)
         d.lin(m + "experts.gate_up_proj", E, 2 * I, H)
-        d.lin(m + "experts.down_proj", E, H, I)
+        d.lin(m + "experts.down_proj", E, H, I, gain=DOWN)
         d.lin(m + "shared_expert.up_proj.weight", S, H)
         d.lin(m + "shared_expert.gate_proj.weight", S, H)
         d.lin(m + "shared_expert.down_proj.weight", H, S)
@@ -236,7 +236,7 @@ def _hybrid_weights(d, c):
 def _experts(d, m, n, ff, W, gated):
     """Expert by expert, as checkpoints name them (views of one draw)."""
     for part, shape in (("up", (n, ff, W)), ("down", (n, W, ff))) + ((("gate", (n, ff, W)),) if gated else ()):
-        d.lin("stack", *shape)
+        d.lin("stack", *shape, gain=DOWN if part == "down" else 1.0)
         for j, t in enumerate(d.t.pop("stack")):
             d.t[m + f"e{j}.{part}"] = t
 
@@ -401,7 +401,7 @@ def _nopuzen_weights(d, c):
             d.lin(m + "down", W, L.ff)
             d.around(m + "act", 2, -1.0, 0.3)
         else:
-            d.lin(m + "router", e.experts, W, gain=ROUTER)
+            d.lin(m + "router", e.experts, W, gain=ROUTER / 3)      # reads the stream itself, which is about 3 wide
             _experts(d, m, e.experts, e.ff, W, False)
             d.lin(m + "shared.up", e.shared_ff, W)
             d.lin(m + "shared.down", W, e.shared_ff)
@@ -629,8 +629,8 @@ def work(case):
 
 
 def tolerance(case):
-    """bf16 operands through a few layers, against 64 bits: 0.0034 for the video block, 0.004 - 0.007 for decoders, up
-    to 0.025 where a token whose last expert hangs on rounding takes another one, or where experts are FP8; single
+    """bf16 operands through a few layers, against 64 bits: 0.0034 for the video block, 0.003 - 0.007 for decoders, up
+    to 0.016 where a token whose last expert hangs on rounding takes another one, or where experts are FP8; single
     values of such a token's row move by more."""
     if case["model"] == "h3":
         return {"rel": 0.013, "max": 0.3}
