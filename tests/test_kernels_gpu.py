@@ -783,6 +783,45 @@ def test_gated_delta_rule_kernel(Dk, Dv, Hk, Hv, dtype):
     tol.check(S2, ref_S, "state vs the chunked form")
 
 
+@pytest.mark.parametrize("Dk,Dv,Hk,Hv,K,lens,dtype", [
+    (128, 128, 2, 4, 4, [16, 67], BF), (36, 20, 2, 2, 2, [131], torch.float32), (64, 132, 1, 3, 3, [2, 33, 13], BF)])
+def test_hybrid_mixer_rows(Dk, Dv, Hk, Hv, K, lens, dtype):
+    """Preparation and four-token recurrence of the hybrid layers' prompts (fewer rows than taps, blocks and tiles that
+    end in between, widths past 128) against convolution, gates and the stepwise recurrence in FP32."""
+    from uniserve_v1_b200.ops import gated_delta as GD
+    T, B, C, rep = sum(lens), len(lens), 2 * Hk * Dk + Hv * Dv, Hv // Hk
+    pad = -(C + 2 * Hv) % 4
+    x = rnd(T, C + 2 * Hv + pad, dtype=dtype, seed=1)
+    offs = (0, Hk * Dk, 2 * Hk * Dk, C, C + Hv)
+    w, A, bias = rnd(C, K, dtype=torch.float32, scale=0.5, seed=2), -(torch.rand(Hv, device=DEV) + 0.2), rnd(
+        Hv, dtype=torch.float32, seed=3)
+    conv0, pool0 = rnd(B + 1, K - 1, C, dtype=dtype, seed=4), rnd(B + 1, Hv, Dk, Dv, dtype=torch.float32, scale=0.1, seed=5)
+    conv, pool = conv0.clone(), pool0.clone()
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    slots = torch.arange(B, 0, -1, dtype=torch.int32, device=DEV)
+    assert GD.mixer_serves(x, K, offs, Hv, Dk, Dv, T, B) == (T >= 16 * B)
+    out = GD.mixer_rows(x, offs, w, conv, A, bias, pool, cu, slots, Hk, Hv, Dk, Dv)
+    # as for the recurrence alone; a convolved value that stands between two bf16 values may take the other one
+    tol = Tolerance.dot(Dk, out=torch.float32).then(Tolerance(0.0, 2.0 ** -19, True)).scaled(max(lens))
+    if dtype == BF:
+        tol = tol.then(Tolerance(0.0, 2.0 ** -9, True))
+    xc, lo = x.float().cpu(), 0
+    for n, s in zip(lens, slots.tolist()):
+        sl = slice(lo, lo + n)
+        y, state = GD.causal_conv1d(xc[sl, :C], w.cpu(), conv0[s].float().cpu())
+        y = y.to(dtype).float()                  # the convolved rows have the projection's type
+        q, k, v = torch.split(y, [Hk * Dk, Hk * Dk, Hv * Dv], 1)
+        q, k = (t.reshape(n, Hk, Dk).repeat_interleave(rep, 1) for t in (q, k))
+        g = A.cpu() * torch.nn.functional.softplus(xc[sl, offs[4]:offs[4] + Hv] + bias.cpu())
+        ref_o, ref_S = GD.gated_delta_rule_steps(q, k, v.reshape(n, Hv, Dv), g, torch.sigmoid(xc[sl, C:C + Hv]),
+                                                 pool0[s].cpu())
+        tol.check(out[sl], ref_o, "hybrid mixer output")
+        tol.check(pool[s], ref_S, "hybrid mixer state")
+        Tolerance.exact().check(conv[s], state.to(dtype), "hybrid mixer window")
+        lo += n
+    Tolerance.exact().check(pool[0], pool0[0], "untouched slot")
+
+
 def test_rmsnorm_gated_kernel():
     from uniserve_v1_b200.ops import gated_delta as GD
     T, Hv, Dv = 19, 8, 128

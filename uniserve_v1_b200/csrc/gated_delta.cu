@@ -259,6 +259,61 @@ rmsnorm_gated_kernel(const float* __restrict__ x, const void* __restrict__ w,
   }
 }
 
+// The same for heads in fours: a lane owns four neighbouring columns, NG such groups (16-byte loads of x, 8-byte ones
+// of bf16 weights and gates).  4093 rows of 32 heads of 128: 56 -> 40 us (read once, written once: 20).
+template <int NG, bool BF>
+__global__ void __launch_bounds__(256)
+rmsnorm_gated_quad_kernel(const float* __restrict__ x, const void* __restrict__ w, const void* __restrict__ z, long long ldz,
+                          int hsz, void* __restrict__ y, int rows, int Hv, int Dv, float eps) {
+  US_PDL_PROLOGUE();
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  const int t = r / Hv, h = r - t * Hv;
+  auto rnd = [](float v) { return BF ? us::bf2f(us::f2bf(v)) : v; };
+  auto quad = [](const void* base, long long at, float (&o)[4]) {
+    if (BF) {
+      us::Pack8 p;
+      p.u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(base) + at);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = us::bf2f(p.b[e]);
+    } else {
+      const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + at);
+      o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+    }
+  };
+  float xv[NG][4], g[NG][4], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NG; ++i) {
+    const int d = i * 128 + lane * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) xv[i][e] = g[i][e] = 0.f;
+    if (d >= Dv) continue;
+    const float4 v = *reinterpret_cast<const float4*>(x + (long long)r * Dv + d);
+    xv[i][0] = rnd(v.x); xv[i][1] = rnd(v.y); xv[i][2] = rnd(v.z); xv[i][3] = rnd(v.w);
+    quad(z, (long long)t * ldz + (long long)h * hsz + d, g[i]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ss += xv[i][e] * xv[i][e];
+  }
+  const float inv = rsqrtf(us::warp_sum(ss) / (float)Dv + eps);
+#pragma unroll
+  for (int i = 0; i < NG; ++i) {
+    const int d = i * 128 + lane * 4;
+    if (d >= Dv) continue;
+    float wv[4], o[4];
+    quad(w, d, wv);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = rnd(rnd(xv[i][e] * inv) * wv[e]) * silu(g[i][e]);
+    if (BF) {
+      us::Pack8 p;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p.b[e] = us::f2bf(o[e]);
+      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(y) + (long long)r * Dv + d) = p.u;
+    } else {
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + (long long)r * Dv + d) = make_float4(o[0], o[1], o[2], o[3]);
+    }
+  }
+}
+
 }  // namespace
 
 US_API int us_causal_conv1d(const void* x, long long ldx, const void* w, void* state, void* y,
@@ -304,6 +359,23 @@ US_API int us_gated_delta_rule(const void* q, const void* k, const void* v, long
 US_API int us_rmsnorm_gated(const float* x, const void* w, const void* z, long long ldz, int hsz,
                             void* y, int rows, int Hv, int Dv, float eps, int bf16, void* stream_) {
   US_REQUIRE(x && w && z && y && rows >= 1 && Hv >= 1 && Dv >= 1);
+  const size_t piece = bf16 ? 8 : 16;
+  if ((Dv & 3) == 0 && Dv <= 256 && (ldz & 3) == 0 && (hsz & 3) == 0 && ((uintptr_t)x % 16) == 0 &&
+      (((uintptr_t)w | (uintptr_t)z | (uintptr_t)y) % piece) == 0) {
+    const dim3 grid((rows + 7) / 8), block(256);
+    cudaStream_t stream = (cudaStream_t)stream_;
+#define US_GATED(NG, BF) \
+  US_CUDA_CHECK(us::launch_pdl(rmsnorm_gated_quad_kernel<NG, BF>, grid, block, 0, stream, x, w, z, ldz, hsz, y, rows, Hv, Dv, eps))
+    if (bf16) {
+      if (Dv <= 128) US_GATED(1, true);
+      else US_GATED(2, true);
+    } else {
+      if (Dv <= 128) US_GATED(1, false);
+      else US_GATED(2, false);
+    }
+#undef US_GATED
+    return US_OK;
+  }
   US_CUDA_CHECK(us::launch_pdl(rmsnorm_gated_kernel, dim3((rows + 7) / 8), dim3(256), 0,
                                (cudaStream_t)stream_, x, w, z, ldz, hsz, y, rows, Hv, Dv, eps, bf16));
   return US_OK;

@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, DP > 128 ? 1 : 2) head_delta_kernel(
   const int own = kq >> 2, mine_t = kq & 3;           // its own column; the token whose read-out it finishes
   const int cb = warp * 8 + (lane >> 4) * 4;
   float* Sg = a.state + ((long long)slot * a.H + h) * a.D * a.V;
-  const bool fresh = a.pos[start] == 0;
+  const bool fresh = a.pos && a.pos[start] == 0;
   // the c-th column of a lane is cb + (own ^ c): what it holds for others, they hold for it at the same c
   f2 S[NG * 2][4];                                    // row pairs x columns
 #pragma unroll
@@ -378,12 +378,12 @@ US_API long long us_head_delta_coef_floats(int rows, int B, int H) {
 }
 
 // q and k heads serve H / Hk value heads each; all vectors dense FP32; coef: scratch of
-// us_head_delta_coef_floats floats.
+// us_head_delta_coef_floats floats; pos null: every sequence goes on from its slot's state.
 US_API int us_head_delta_rule(const float* q, const float* k, const float* v, const float* g,
                               const float* beta, float* coef, float* state, float* out, const int* cu,
                               const int* slots, const int* pos, int B, int rows, int H, int Hk, int D, int V,
                               void* stream_) {
-  US_REQUIRE(q && k && v && g && beta && coef && state && out && cu && slots && pos && B >= 1 && B <= 65535);
+  US_REQUIRE(q && k && v && g && beta && coef && state && out && cu && slots && B >= 1 && B <= 65535);
   US_REQUIRE(rows >= 0 && H >= 1 && Hk >= 1 && H % Hk == 0 && H <= 65535 && D >= 1 && V >= 1);
   US_REQUIRE(((uintptr_t)coef % 16) == 0);
   US_REQUIRE((D & 3) || (V & 3) || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) % 16) == 0);

@@ -181,6 +181,7 @@ union Pack16 {
 union Pack8 {
   uint2 u;
   __nv_bfloat16 b[4];
+  __nv_bfloat162 b2[2];
 };
 
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }

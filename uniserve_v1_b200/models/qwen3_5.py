@@ -274,6 +274,17 @@ class Qwen35MoeModel:
         proj = F.linear(n, L["qkvz"])
         mixed, z = proj[:, :2 * kd + vd], proj[:, 2 * kd + vd:2 * kd + 2 * vd]
         b, a = proj[:, 2 * kd + 2 * vd:2 * kd + 2 * vd + Hv], proj[:, 2 * kd + 2 * vd + Hv:]
+        offs, K = (0, kd, 2 * kd, 2 * kd + 2 * vd, 2 * kd + 2 * vd + Hv), L["conv"].shape[1]
+        if GD.mixer_serves(proj, K, offs, Hv, Dk, Dv, T, 1):
+            if st.rule is None:
+                st.rule = torch.zeros(Hv, Dk, Dv, dtype=torch.float32, device=n.device)
+            st.conv = torch.zeros(K - 1, 2 * kd + vd, dtype=n.dtype, device=n.device) if st.conv is None \
+                else st.conv.to(n.dtype).clone()
+            cu, slots = GD._one_sequence(T, n.device)
+            o = GD.mixer_rows(proj, offs, L["conv"].float().contiguous(), st.conv.unsqueeze(0), L["A"].float().contiguous(),
+                              L["dt_bias"].float().contiguous(), st.rule.unsqueeze(0), cu, slots, Hk, Hv, Dk, Dv)
+            o = GD.rmsnorm_gated(o, L["gnorm"], z.unflatten(1, (Hv, Dv)), c.rms_norm_eps)
+            return F.linear(o.reshape(T, vd), L["out"])
         if n.is_cuda and GD.USE_KERNELS and Dk in GD._KERNEL_DK:
             # kernels: the convolution reads the projection in place, the rule reads q / k / v
             # as views of the convolved rows (a key head serves Hv / Hk value heads) and forms

@@ -113,6 +113,38 @@ def gated_delta_rule_packed(q, k, v, state, cu, slots, g=None, beta=None, raw=No
     return out
 
 
+# Rows per sequence from which the hybrid layers run the four-token recurrence behind one preparation launch; below,
+# its scratch and two more launches cost as much as the recurrence token by token (0.73 us a token and sequence).
+MIXER_MIN_ROWS = 16
+
+
+def mixer_serves(x, K: int, offs, Hv: int, Dk: int, Dv: int, rows: int, sequences: int) -> bool:
+    """Whether ``mixer_rows`` runs these sizes: widths and columns in fours, up to four taps, enough rows."""
+    return USE_KERNELS and x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and x.stride(1) == 1 and \
+        2 <= K <= 4 and not any(n % 4 for n in (Dk, Dv, x.stride(0), *offs[:3])) and max(Dk, Dv) <= 256 and \
+        x.data_ptr() % (8 if x.dtype == torch.bfloat16 else 16) == 0 and rows >= MIXER_MIN_ROWS * sequences
+
+
+def mixer_rows(x, offs, conv_w, conv, A, dt_bias, state, cu, slots, Hk: int, Hv: int, Dk: int, Dv: int):
+    """Convolution, unit q / k, gates and the rule of projection rows ``x`` [T, .] (GPU, ``mixer_serves``): q, k, v, b
+    and a stand at the columns ``offs``.  ``conv`` [n, K - 1, C] and ``state`` [n, Hv, Dk, Dv] are updated in place for
+    the sequences ``slots`` whose rows are ``cu``.  Vectors and recurrence in FP32; returns o [T, Hv, Dv] FP32."""
+    T, B, K, nq = x.shape[0], slots.shape[0], conv_w.shape[1], Hk * Dk
+    f = dict(dtype=torch.float32, device=x.device)
+    q, k, v = torch.empty(T, Hk, Dk, **f), torch.empty(T, Hk, Dk, **f), torch.empty(T, Hv, Dv, **f)
+    g, beta, out = torch.empty(T, Hv, **f), torch.empty(T, Hv, **f), torch.empty(T, Hv, Dv, **f)
+    coef = torch.empty(N.kernels().us_head_delta_coef_floats(T, B, Hv), **f)
+    for t in (conv_w, conv, A, dt_bias, state):
+        assert t.is_contiguous()
+    assert conv_w.dtype == A.dtype == dt_bias.dtype == state.dtype == torch.float32 and conv.dtype == x.dtype
+    N.call("us_window_delta_prep", N.ptr(x), x.stride(0), *offs, N.ptr(conv_w), N.ptr(conv_w[nq:]), N.ptr(conv_w[2 * nq:]),
+           N.ptr(A), N.ptr(dt_bias), N.ptr(conv), N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(g), N.ptr(beta), N.ptr(cu),
+           N.ptr(slots), B, T, Hv, Hk, Dk, Dv, K, int(x.dtype == torch.bfloat16), N.stream(), launches=2)
+    N.call("us_head_delta_rule", N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(g), N.ptr(beta), N.ptr(coef), N.ptr(state),
+           N.ptr(out), N.ptr(cu), N.ptr(slots), None, B, T, Hv, Hk, Dk, Dv, N.stream(), launches=2)
+    return out
+
+
 def gated_delta_rule_chunked(q, k, v, g, beta, state=None, chunk: int = 64):
     """The same recurrence, C positions at a time.  With G the running sum of g inside
     the chunk and S0 the state at its start, the corrections u_t = beta_t (v_t - S_{t-1}^T k_t)

@@ -53,6 +53,7 @@ _SIGNATURES = {
                                   F, I, I, P]),
     "us_head_delta_prep": (I, [P, L, I, I, I, I, I, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I,
                                I, I, I, I, I, P]),
+    "us_window_delta_prep": (I, [P, L, I, I, I, I, I, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P]),
     "us_head_delta_coef_floats": (L, [I, I, I]),
     "us_head_delta_rule": (I, [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P]),
     "us_head_delta_step": (I, [P, L, I, I, I, I, I, P, P, P, P, P, P, P, P, I, P, L, P, L, P, P, I, I, I,
