@@ -45,19 +45,19 @@ NVCC_FLAGS = [
 GROUPS = {
     "nepevik": (("runtime.cu", "gemm_tc05.cu", "linear_decode.cu", "gemm_f32.cu", "moe_route.cu",
                  "misc.cu", "sampler.cu", "row_ops.cu", "vector_delta.cu", "head_mix_attn.cu"),
-                ("block_manager.cpp",)),
+                ("block_manager.cpp", "batch_rows.cpp")),
     "zonopel": (("runtime.cu", "gemm_tc05.cu", "linear_decode.cu", "gemm_f32.cu", "misc.cu", "sampler.cu",
                  "stream_rows.cu", "state_space.cu", "state_space_chunk.cu", "latent_attn.cu", "latent_decode.cu",
                  "latent_flash_tc05.cu"),
-                ("block_manager.cpp",)),
+                ("block_manager.cpp", "batch_rows.cpp")),
     "tadinex": (("runtime.cu", "gemm_tc05.cu", "linear_decode.cu", "gemm_f32.cu", "moe_route.cu", "misc.cu",
                  "sampler.cu", "stream_rows.cu", "vector_delta.cu", "head_delta.cu", "state_space.cu",
                  "state_space_chunk.cu", "window_attn.cu", "latent_flash_tc05.cu", "attn_decode.cu", "attn_decode_tc05.cu"),
-                ("block_manager.cpp",)),
+                ("block_manager.cpp", "batch_rows.cpp")),
     "nopuzen": (("runtime.cu", "gemm_tc05.cu", "linear_decode.cu", "gemm_f32.cu", "moe_route.cu", "misc.cu",
                  "sampler.cu", "stream_rows.cu", "latent_attn.cu", "latent_decode.cu", "latent_flash_tc05.cu",
                  "window_attn.cu", "sigmoid_decode.cu"),
-                ("block_manager.cpp",)),
+                ("block_manager.cpp", "batch_rows.cpp")),
 }
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-pthread", "-Wall"]
 

@@ -15,6 +15,8 @@ project paths.
 """
 from __future__ import annotations
 
+import ctypes
+from array import array
 from dataclasses import dataclass, field
 from typing import Optional
 
@@ -322,15 +324,16 @@ class CausalLmRunner:
                 self._graph(B, v)
 
     # ---------------------------------------------------------------- decode --
-    def _fill_decode(self, blk: InputBlock, rows: list, B: int) -> None:
+    def _fill_decode(self, blk: InputBlock, rows: list, B: int, variant: str = "sampled") -> None:
         """Column assembly of a decode batch into the pinned input block (numpy
-        views over the pinned memory; one pass over the rows)."""
+        views over the pinned memory; one pass over the rows).  Only a ``sampled`` step
+        reads the sampler's columns: others leave them as they are."""
         h = blk.hn
         n = len(rows)
         ps = self.page_size
         h["live"][0] = n
         h["step"][0] = 0
-        ids, pos, slots, temp, top_k, top_p, min_p, seeds = [], [], [], [], [], [], [], []
+        ids, pos, slots = [], [], []
         pt = h["page_table"]
         # A row of the page table is rewritten only when its request or its page list
         # changed; a list that grew gets its new tail (page lists only ever append, and a
@@ -350,6 +353,22 @@ class CausalLmRunner:
             else:
                 pt[i, :n_p] = pages
             held[i] = (pages, n_p)
+        h["input_ids"][:n] = ids
+        h["positions"][:n] = pos
+        h["seq_lens"][:n] = pos
+        h["seq_lens"][:n] += 1
+        h["slots"][:n] = slots
+        h["state_slots"][:n] = [req.slot for req in rows]
+        if n < B:
+            h["input_ids"][n:] = 0
+            h["positions"][n:] = 0
+            h["seq_lens"][n:] = 0
+            h["slots"][n:] = -1
+            h["state_slots"][n:] = -1
+        if variant != "sampled":
+            return
+        temp, top_k, top_p, min_p, seeds = [], [], [], [], []
+        for req in rows:
             p: SamplingParams = req.params
             greedy = p.greedy
             temp.append(1.0 if greedy else p.temperature)
@@ -358,12 +377,6 @@ class CausalLmRunner:
             min_p.append(p.min_p)
             sd = req.seed
             seeds.append(sd - (1 << 64) if sd >= (1 << 63) else sd)
-        h["input_ids"][:n] = ids
-        h["positions"][:n] = pos
-        h["seq_lens"][:n] = pos
-        h["seq_lens"][:n] += 1
-        h["slots"][:n] = slots
-        h["state_slots"][:n] = [req.slot for req in rows]
         h["temperature"][:n] = temp
         h["top_k"][:n] = top_k
         h["top_p"][:n] = top_p
@@ -372,11 +385,6 @@ class CausalLmRunner:
         h["sample_pos"][:n] = pos
         h["sample_pos"][:n] += 1
         if n < B:
-            h["input_ids"][n:] = 0
-            h["positions"][n:] = 0
-            h["seq_lens"][n:] = 0
-            h["slots"][n:] = -1
-            h["state_slots"][n:] = -1
             h["temperature"][n:] = 1.0
             h["top_k"][n:] = 1
             h["top_p"][n:] = 1.0
@@ -458,7 +466,7 @@ class CausalLmRunner:
         variant = self.variant_for(rows) if rows else "greedy"
         assert steps == 1 or variant != "logits"
         assert steps <= self.history_steps
-        self._fill_decode(blk, rows, B)
+        self._fill_decode(blk, rows, B, variant)
         g = self._graph(B, variant) if B <= self.buckets[-1] or B in self._graphs else None
         self.h2d_bytes += blk.upload()
         logits = sampled = None
@@ -498,7 +506,7 @@ class CausalLmRunner:
         blk = self._decode_block(B)
         variant = self.variant_for(rows)
         assert variant != "logits"
-        self._fill_decode(blk, rows, B)
+        self._fill_decode(blk, rows, B, variant)
         g = self._graph(B, variant) if B <= self.buckets[-1] or B in self._graphs else None
         self.h2d_bytes += blk.upload()
         return DecodeStream(rows=list(rows), n=n, B=B, blk=blk, graph=g, variant=variant)
@@ -529,6 +537,11 @@ class CausalLmRunner:
             self.d2h_bytes += st.n * 4 + 4
             return st.blk.readback[k, :st.n].tolist()
         return st.blk.history[k, :st.n].tolist()
+
+    def _row_index(self, rows: list) -> torch.Tensor:
+        """Row numbers on the device, without waiting for what runs there (a copy from pageable memory does)."""
+        pin = self.device.type == "cuda"
+        return torch.tensor(rows, dtype=torch.int32, pin_memory=pin).to(self.device, non_blocking=True)
 
     def _to_host(self, t: torch.Tensor) -> torch.Tensor:
         host = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
@@ -654,9 +667,7 @@ class CausalLmRunner:
         sample_rows = [c.request for c in chunks if c.sample]
         if not sample_rows:
             return None, None, []
-        rows_idx = torch.tensor(last_rows, dtype=torch.int32, device=dev)
-        last = F.gather_rows(hidden, rows_idx)
-        logits = self.model.logits(last)
+        logits = self.model.logits(F.gather_rows(hidden, self._row_index(last_rows)))
         if self.variant_for(sample_rows) == "greedy":
             toks = F.argmax(logits)
             host = self._to_host(toks) if dev.type == "cuda" else toks
@@ -673,7 +684,7 @@ class CausalLmRunner:
             rows = [c.request for c in batch.chunks]
             B = self.bucket_for(len(rows))
             blk = self._decode_block(B)
-            self._fill_decode(blk, rows, B)
+            self._fill_decode(blk, rows, B, "logits")
             g = self._graph(B, "logits")
             self.h2d_bytes += blk.upload()
             if g is not None:
@@ -683,12 +694,16 @@ class CausalLmRunner:
             else:
                 logits, _ = self._decode_body(blk, B, "logits")
             idx = [i for i, w in enumerate(want) for _ in w]
-            logits = logits[torch.tensor(idx, dtype=torch.long, device=dev)] if idx else None
+            if not idx:
+                logits = None
+            elif idx == list(range(len(idx))):          # every row once: no copy of them
+                logits = logits[:len(idx)]
+            else:
+                logits = logits[self._row_index(idx)]
         else:
             hidden, cu_q = self._prefill_rows(batch.chunks)
             idx = [cu_q[i] + j for i, w in enumerate(want) for j in w]
-            logits = self.model.logits(F.gather_rows(
-                hidden, torch.tensor(idx, dtype=torch.int32, device=dev))) if idx else None
+            logits = self.model.logits(F.gather_rows(hidden, self._row_index(idx))) if idx else None
         if dev.type != "cuda":
             return logits
         if logits is None:
@@ -701,46 +716,42 @@ class CausalLmRunner:
     def _prefill_rows(self, chunks: list, capacity: Optional[int] = None):
         """The forward of ``prefill``: (hidden rows, row offset of every chunk)."""
         dev = self.device
-        ps = self.page_size
-        ids, pos, slots, cu_q, cu_k, ctx = [], [], [], [0], [0], []
-        max_q = max_k = 0
+        ctx = [c.start for c in chunks]
+        q_lens = [c.length for c in chunks]
+        cu_q, cu_k, ids, held = [0], [0], [], []
         for c in chunks:
-            req = c.request
-            toks = req.all_ids[c.start:c.start + c.length]
-            ids.extend(toks)
-            pos.extend(range(c.start, c.start + c.length))
-            for p_ in range(c.start, c.start + c.length):
-                slots.append(req.pages[p_ // ps] * ps + p_ % ps)
             cu_q.append(cu_q[-1] + c.length)
             cu_k.append(cu_k[-1] + c.start + c.length)
-            ctx.append(c.start)
-            max_q = max(max_q, c.length)
-            max_k = max(max_k, c.start + c.length)
-        T_real = len(ids)
-        live = None
-        if capacity is not None:
-            assert T_real <= capacity, (T_real, capacity)
-            pad = capacity - T_real
-            ids, pos, slots = ids + [0] * pad, pos + [0] * pad, slots + [-1] * pad
-            live = torch.tensor([T_real], dtype=torch.int32, device=dev)
-        T = len(ids)
-        i32 = torch.int32
-        packed = torch.tensor(ids + pos + slots + cu_q + cu_k + [c.request.slot for c in chunks],
-                              dtype=i32, pin_memory=dev.type == "cuda")
+            ids += c.request.token_slice(c.start, c.start + c.length)
+            held += c.request.pages
+        max_q = max(q_lens, default=0)
+        max_k = max((a + n for a, n in zip(ctx, q_lens)), default=0)
+        T_real = cu_q[-1]
+        assert len(ids) == T_real, (len(ids), T_real)
+        assert capacity is None or T_real <= capacity, (T_real, capacity)
+        T = T_real if capacity is None else capacity
+        nq, B = len(cu_q), len(chunks)
+        tables = self.attends_pages or any(a > 0 for a in ctx)
+        # one pinned buffer, one copy; the page table starts on 16 bytes
+        at = 3 * T + 2 * nq + B + 1
+        first = -(-at // 4) * 4
+        packed = torch.empty(first + (B * self.max_pages if tables else 0), dtype=torch.int32,
+                             pin_memory=dev.type == "cuda")
+        plan = array("i", ctx + q_lens + [len(c.request.pages) for c in chunks] +
+                     [c.request.slot for c in chunks] + held)
+        ids = array("i", ids)
+        bad = N.host().us_batch_rows(*(ctypes.c_void_p(x.buffer_info()[0]) for x in (plan, ids)), B, T,
+                                     self.page_size, self.max_pages if tables else 0, first, N.ptr(packed))
+        if bad:
+            raise IndexError(f"request {chunks[bad - 1].request.request_id}: its pages do not hold its tokens")
         d = packed.to(dev, non_blocking=True)
         self.h2d_bytes += packed.numel() * 4
-        nq = len(cu_q)
-        page_table = None
-        if self.attends_pages or any(c > 0 for c in ctx):
-            page_table = torch.zeros(len(chunks), self.max_pages, dtype=i32)
-            for i, c in enumerate(chunks):
-                page_table[i, :len(c.request.pages)] = torch.tensor(c.request.pages, dtype=i32)
-            page_table = page_table.to(dev)
+        page_table = d[first:].view(B, self.max_pages) if tables else None
         meta = AttnMeta(kind="prefill", slots=d[2 * T:3 * T], cu_q=d[3 * T:3 * T + nq],
                         cu_k=d[3 * T + nq:3 * T + 2 * nq], max_q=max_q, max_k=max_k,
-                        context_lens=ctx, q_lens=[c.length for c in chunks], page_table=page_table,
-                        live=live, rows_real=T_real,
-                        state_slots=d[3 * T + 2 * nq:], states=self.states)
+                        context_lens=ctx, q_lens=q_lens, page_table=page_table,
+                        live=d[at - 1:at] if capacity is not None else None, rows_real=T_real,
+                        state_slots=d[3 * T + 2 * nq:at - 1], states=self.states)
         if page_table is not None and dev.type == "cuda" and not self.attends_pages:
             from ..ops.attention import context_tables
             meta.ctx_tables = context_tables(ctx, cu_q, cu_k, dev)

@@ -95,14 +95,14 @@ def context_tables(ctx: list, cu_q: list, cu_k: list, device):
     scheduler's host-side plan): cumulative context lengths [B + 1] (int32), the row of every
     new key in the combined per-sequence [cached; new] buffer [T] (int64), and the total
     number of cached rows."""
-    ctx_cu, new_dst = [0], []
+    pin = torch.device(device).type == "cuda"
+    ctx_cu = [0]
+    new_dst = torch.empty(cu_q[-1], dtype=torch.int64, pin_memory=pin)
     for i, c in enumerate(ctx):
         ctx_cu.append(ctx_cu[-1] + c)
-        n = cu_q[i + 1] - cu_q[i]
-        new_dst.extend(range(cu_k[i] + c, cu_k[i] + c + n))
-    pin = torch.device(device).type == "cuda"
+        torch.arange(cu_k[i] + c, cu_k[i] + c + cu_q[i + 1] - cu_q[i], out=new_dst[cu_q[i]:cu_q[i + 1]])
     a = torch.tensor(ctx_cu, dtype=torch.int32, pin_memory=pin).to(device, non_blocking=True)
-    b = torch.tensor(new_dst, dtype=torch.int64, pin_memory=pin).to(device, non_blocking=True)
+    b = new_dst.to(device, non_blocking=True)
     return a, b, ctx_cu[-1]
 
 

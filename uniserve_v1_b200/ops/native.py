@@ -208,7 +208,9 @@ def ptr(t):
 
 
 def stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream.  Asked of the binding itself: ``torch.cuda.current_stream()`` builds an object and
+    looks its device up, 5 us of the 20 that a launch from Python took; a prompt of 200 tokens waits for launches."""
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def check(rc: int, what: str = "") -> None:
