@@ -29,6 +29,7 @@ import torch
 
 from ..ops import functional as F
 from ..ops import gated_delta as GD
+from ..ops import hybrid_rows as HR
 from ..ops import reference as R
 
 
@@ -117,6 +118,12 @@ class SequenceState(list):
     mtp = None
 
 
+def _join_qkv(L: dict) -> None:
+    """One projection for queries (with their gates), keys and values; its parts stay as views."""
+    L["qkv"] = torch.cat([L["q"], L["k"], L["v"]], 0)
+    L["q"], L["k"], L["v"] = L["qkv"].split([L[n].shape[0] for n in "qkv"])
+
+
 class Qwen35MoeModel:
     def __init__(self, cfg: Qwen35Config, device="cpu", dtype=torch.bfloat16):
         self.cfg, self.device, self.dtype = cfg, torch.device(device), dtype
@@ -147,6 +154,7 @@ class Qwen35MoeModel:
             if kind == "full_attention":
                 a = p + "self_attn."
                 L["q"], L["k"], L["v"], L["o"] = (get(a + f"{n}_proj.weight") for n in "qkvo")
+                _join_qkv(L)
                 L["q_norm"] = get(a + "q_norm.weight", torch.float32) + 1.0
                 L["k_norm"] = get(a + "k_norm.weight", torch.float32) + 1.0
             else:
@@ -212,6 +220,7 @@ class Qwen35MoeModel:
                 L["q"] = rnd(c.num_attention_heads * 2 * D, H)
                 L["k"], L["v"] = rnd(c.num_key_value_heads * D, H), rnd(c.num_key_value_heads * D, H)
                 L["o"] = rnd(H, c.num_attention_heads * D)
+                _join_qkv(L)
                 L["q_norm"], L["k_norm"] = ones(D), ones(D)
             else:
                 L["qkvz"] = rnd(2 * kd + 2 * vd + 2 * c.linear_num_value_heads, H)
@@ -248,6 +257,15 @@ class Qwen35MoeModel:
         c, D = self.cfg, self.cfg.head_dim
         T = n.shape[0]
         Hq, Hkv = c.num_attention_heads, c.num_key_value_heads
+        if "qkv" in L and pos3 is None and HR.heads_serve(n, D):
+            proj = F.linear(n, L["qkv"])
+            q, k, v = HR.heads(proj, L["q_norm"], L["k_norm"], self.inv_freq, pos0, Hq, Hkv, D, self.rot,
+                               c.rms_norm_eps)
+            att = self._attend(q, k, v, st)
+            if att.dtype == proj.dtype:
+                return F.linear(HR.gate(att.reshape(T, Hq * D), proj, Hq, D), L["o"])
+            gate = proj[:, :2 * Hq * D].view(T, Hq, 2 * D)[..., D:].reshape(T, Hq * D)
+            return F.linear((att.reshape(T, Hq * D) * torch.sigmoid(gate.float())).to(n.dtype), L["o"])
         qg = F.linear(n, L["q"]).view(T, Hq, 2 * D)
         q, gate = qg[..., :D], qg[..., D:].reshape(T, Hq * D)
         k = F.linear(n, L["k"]).view(T, Hkv, D)
@@ -258,12 +276,15 @@ class Qwen35MoeModel:
                                   self.rot, False, c.rms_norm_eps)
         else:
             q, k = self._norm_mrope(q, L["q_norm"], pos3), self._norm_mrope(k, L["k_norm"], pos3)
+        att = self._attend(q, k, v, st).reshape(T, Hq * D)
+        att = (att * torch.sigmoid(gate.float())).to(n.dtype)
+        return F.linear(att, L["o"])
+
+    def _attend(self, q, k, v, st: LayerState):
         st.k = k if st.k is None else torch.cat([st.k, k], 0)
         st.v = v if st.v is None else torch.cat([st.v, v], 0)
         from ..ops.attention import cached_causal_attention
-        att = cached_causal_attention(q, st.k, st.v, 1.0 / math.sqrt(D)).reshape(T, Hq * D)
-        att = (att * torch.sigmoid(gate.float())).to(n.dtype)
-        return F.linear(att, L["o"])
+        return cached_causal_attention(q, st.k, st.v, 1.0 / math.sqrt(self.cfg.head_dim))
 
     def _linear_attention(self, L, n, st: LayerState):
         c = self.cfg
@@ -322,6 +343,17 @@ class Qwen35MoeModel:
         sg = torch.sigmoid(F.linear(n, L["sgate"], out_dtype=torch.float32))
         return y + (shared.float() * sg).to(n.dtype)
 
+    def _mlp_output(self, L, n, shared_gate) -> HR.Output:
+        """``_mlp`` up to its sums, which ``HR.add_norm`` forms with the residual and the next norm."""
+        c = self.cfg
+        if "d13" in L:
+            return HR.Output(rows=F.linear(F.linear_gated(n, L["d13"]), L["d2"]))
+        logits = F.linear(n, L["router"], out_dtype=torch.float32)
+        ids, wts = F.topk_softmax(logits, c.num_experts_per_tok, True)
+        y, perm = F.moe_experts(n, ids, wts, L["w13"], L["w2"], defer_unpermute=True)
+        shared = F.linear(F.linear_gated(n, L["s13"]), L["s2"])
+        return HR.Output(routed=y, perm=perm, weights=wts, shared=shared, shared_gate=shared_gate)
+
     def forward(self, ids: torch.Tensor, state: list, pos0: int = 0, embeds=None,
                 positions3=None, deepstack=None) -> torch.Tensor:
         """Runs ``ids`` [T] at positions pos0 .. on top of ``state``; returns FP32 logits
@@ -331,6 +363,20 @@ class Qwen35MoeModel:
         c, w = self.cfg, self.w
         x = w["embed"][ids.to(self.device).long()] if embeds is None else \
             embeds.to(device=self.device, dtype=self.dtype)
+        if HR.rows_serve(x, w["norm"]):
+            eps, out = c.rms_norm_eps, None
+            x = x.contiguous()
+            for i in range(c.num_hidden_layers):
+                L, st = w[i], state[i]
+                x, n, _ = HR.add_norm(x, out, L["in_norm"], eps)
+                mix = self._attention(L, n, st, pos0, positions3) if L["kind"] == "full_attention" \
+                    else self._linear_attention(L, n, st)
+                x, n, shared_gate = HR.add_norm(x, HR.Output(rows=mix), L["post_norm"], eps, L.get("sgate"))
+                out = self._mlp_output(L, n, shared_gate)
+            x, n, _ = HR.add_norm(x, out, w["norm"], eps)
+            if self.tap is not None:
+                self.tap(state, ids, x, pos0)
+            return F.linear(n, w["lm_head"], out_dtype=torch.float32)
         for i in range(c.num_hidden_layers):
             L, st = w[i], state[i]
             n = R.rmsnorm(x, L["in_norm"], c.rms_norm_eps)

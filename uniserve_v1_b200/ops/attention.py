@@ -114,9 +114,8 @@ def cached_causal_attention(q, k_all, v_all, scale):
     T, Hq, D = q.shape
     N_, Hkv = k_all.shape[0], k_all.shape[1]
     if q.is_cuda and q.dtype == BF16 and D % 8 == 0 and D <= 128:
-        dev = q.device
-        cu_q = torch.tensor([0, T], dtype=torch.int32, device=dev)
-        cu_k = torch.tensor([0, N_], dtype=torch.int32, device=dev)
+        from .gated_delta import _one_sequence
+        (cu_q, _), (cu_k, _) = _one_sequence(T, q.device), _one_sequence(N_, q.device)
         q, k_all, v_all = (t if (t.stride(2) == 1 and t.stride(1) == D) else t.contiguous()
                            for t in (q, k_all, v_all))
         return varlen_attention(q, k_all.to(BF16), v_all.to(BF16), cu_q, cu_k, T, N_, scale, True)

@@ -483,6 +483,17 @@ class MoeWorkspace:
             live_tiles=MoeWorkspace._expected_tiles(R_, E_local, E_total or E_local, block_n))
 
     @staticmethod
+    def scratch(T, top_k, E, H, I, device):
+        """For one call with its own sort: nothing in it is read before that call has written it (``create``'s zeros
+        cost nine launches and 26 us at 4093 rows of 2048, four routes each)."""
+        R_ = T * top_k
+        block_n, max_tiles, live = _route_tiles(R_, E, E)
+        ints = torch.empty(2 * R_ + E + 1 + 3 * max_tiles + 1, dtype=torch.int32, device=device)
+        parts = ints.split([R_, R_, E + 1, max_tiles, max_tiles, max_tiles, 1])
+        xp, h, y = (torch.empty(R_, n, dtype=BF16, device=device) for n in (H, I, H))
+        return MoeWorkspace(*parts, xp=xp, h=h, y=y, block_n=block_n, max_tiles=max_tiles, live_tiles=live)
+
+    @staticmethod
     def _expected_tiles(R_, E_local, E_total, block_n) -> int:
         if E_local <= 0:
             return 0
@@ -547,7 +558,7 @@ def moe_experts(x, ids, weights, w13, w2, e_lo=0, act="silu", stepwise=False, ws
     E, I2, _ = w13.shape
     I_ = I2 // 2
     if ws is None:
-        ws = MoeWorkspace.create(T, top_k, E, H, I_, x.device)
+        ws = MoeWorkspace.scratch(T, top_k, E, H, I_, x.device)
     R_ = T * top_k
     st = N.stream()
     if not presorted and not pregathered:

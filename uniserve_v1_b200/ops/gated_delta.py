@@ -25,7 +25,9 @@ USE_KERNELS = True        # False: the PyTorch restatements on every device (A/B
 
 
 def _one_sequence(T: int, device):
-    return (torch.tensor([0, T], dtype=torch.int32, device=device),
+    # counted on the device: a list would be copied from pageable memory, which waits for what runs there
+    return (torch.arange(0, T + 1, max(T, 1), dtype=torch.int32, device=device) if T else
+            torch.zeros(2, dtype=torch.int32, device=device),
             torch.zeros(1, dtype=torch.int32, device=device))
 
 
