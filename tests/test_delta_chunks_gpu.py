@@ -1,0 +1,57 @@
+"""The delta rules sixteen tokens at a time against the token by token recurrence in 64 bits, at the edges of chunks,
+tiles and widths."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(lens, H, Hk, D, V, rate, per_channel):
+    g = torch.Generator(device="cuda").manual_seed(sum(lens) + D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    T = sum(lens)
+    q, k = (torch.nn.functional.normalize(rnd(T, Hk, D) + 0.3, dim=-1) for _ in range(2))
+    shape = (T, H, D) if per_channel else (T, H)
+    decay = torch.exp(-rate * torch.rand(*shape, generator=g, device="cuda"))
+    return q * D ** -0.5, k, rnd(T, H, V), decay, torch.rand(T, H, generator=g, device="cuda"), rnd(len(lens) + 1, H, D, V)
+
+
+def _recurrence(q, k, v, g, beta, S, lens, fresh):
+    q, k, v, g, beta, S = (t.double() for t in (q, k, v, g, beta, S))
+    rep = v.shape[1] // q.shape[1]
+    q, k = q.repeat_interleave(rep, 1), k.repeat_interleave(rep, 1)
+    g = g if g.dim() == 3 else g[:, :, None]
+    out, at = torch.zeros_like(v), 0
+    for s, n in enumerate(lens):
+        if fresh[s]:
+            S[s] = 0
+        for t in range(at, at + n):
+            S[s] *= g[t][:, :, None]
+            u = beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S[s], k[t]))
+            S[s] += k[t][:, :, None] * u[:, None]
+            out[t] = torch.einsum("hdv,hd->hv", S[s], q[t])
+        at += n
+    return out, S
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+@pytest.mark.parametrize("lens,H,Hk,D,V,rate", [
+    ([1], 2, 1, 128, 128, 0.5), ([15, 16, 17], 4, 2, 128, 128, 0.3), ([33, 1, 31], 2, 2, 64, 64, 0.05),
+    ([200], 6, 3, 128, 128, 4.0), ([18, 5], 2, 1, 40, 36, 0.3), ([34], 2, 1, 256, 256, 0.1),
+    ([23, 49], 2, 1, 30, 33, 0.1), ([17], 1, 1, 132, 4, 30.0), ([600], 2, 1, 128, 32, 0.001)])
+def test_chunks_follow_the_recurrence(lens, H, Hk, D, V, rate, per_channel):
+    from uniserve_v1_b200.ops import vector_delta as VD
+    q, k, v, g, beta, S = _inputs(lens, H, Hk, D, V, rate, per_channel)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], **i32)
+    fresh = [i % 2 == 1 for i in range(len(lens))]
+    pos = torch.cat([torch.arange(n, **i32) + (0 if f else 7) for n, f in zip(lens, fresh)])
+    slots = torch.arange(len(lens), **i32)
+    want, state = _recurrence(q, k, v, g, beta, S, lens, fresh)
+    m = VD.SeqMeta(cu, slots, pos, False)
+    got = VD.vector_delta_rule(q, k, v, g, S, m, beta=beta)
+    torch.cuda.synchronize()
+    # FP32 sums of at most D + 16 products, over a few hundred tokens whose state decays: a few times 2^-22 of the norm
+    for a, b in ((got, want), (S, state)):
+        assert float((a.double() - b).norm() / b.norm()) < 2e-6
+    assert torch.equal(S[-1].double(), state[-1])              # a slot that no sequence has

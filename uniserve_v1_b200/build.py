@@ -44,14 +44,14 @@ NVCC_FLAGS = [
 # Sources of the families that can be built alone: (csrc/**.cu, csrc/host/*.cpp).
 GROUPS = {
     "nepevik": (("runtime.cu", "gemm_tc05.cu", "linear_decode.cu", "gemm_f32.cu", "moe_route.cu",
-                 "misc.cu", "sampler.cu", "row_ops.cu", "vector_delta.cu", "head_mix_attn.cu"),
+                 "misc.cu", "sampler.cu", "row_ops.cu", "vector_delta.cu", "chunk_delta.cu", "head_mix_attn.cu"),
                 ("block_manager.cpp", "batch_rows.cpp")),
     "zonopel": (("runtime.cu", "gemm_tc05.cu", "linear_decode.cu", "gemm_f32.cu", "misc.cu", "sampler.cu",
                  "stream_rows.cu", "state_space.cu", "state_space_chunk.cu", "latent_attn.cu", "latent_decode.cu",
                  "latent_flash_tc05.cu"),
                 ("block_manager.cpp", "batch_rows.cpp")),
     "tadinex": (("runtime.cu", "gemm_tc05.cu", "linear_decode.cu", "gemm_f32.cu", "moe_route.cu", "misc.cu",
-                 "sampler.cu", "stream_rows.cu", "vector_delta.cu", "head_delta.cu", "state_space.cu",
+                 "sampler.cu", "stream_rows.cu", "vector_delta.cu", "chunk_delta.cu", "state_space.cu",
                  "state_space_chunk.cu", "window_attn.cu", "latent_flash_tc05.cu", "attn_decode.cu", "attn_decode_tc05.cu"),
                 ("block_manager.cpp", "batch_rows.cpp")),
     "nopuzen": (("runtime.cu", "gemm_tc05.cu", "linear_decode.cu", "gemm_f32.cu", "moe_route.cu", "misc.cu",

@@ -2,7 +2,7 @@
 // a pool.  The decay is a vector over the key channels of a head, or one number per head:
 //
 //   channel rule   S <- diag(g) S;  u = beta (v - S^T k);  S <- S + k u^T;       o = S^T q
-//   head rule      the same with a scalar g (the recurrence itself: head_delta.cu)
+//   head rule      the same with a scalar g
 //   general rule   S <- diag(w) S - (a*n)(n^T S) + k v^T  (both read the old S);  o = S^T q
 //
 // with S [D, V] FP32 per (sequence, head).  The kernels:
@@ -11,7 +11,7 @@
 //                           g = exp(-exp(A_log) softplus(low + dt_bias)) and beta = sigmoid(b)
 //   us_head_delta_prep      the same with the decay's argument a column per head of the projection
 //   us_general_delta_prep   decay w = exp(-c sigmoid(low + w0)), unit key n, removal a * n
-//   us_vector_delta_rule    the recurrence
+//   us_general_delta_rule   the general recurrence (the two others': chunk_delta.cu)
 //   us_head_norm_gate       per-head RMS norm of o, weight, sigmoid or silu gate
 //   us_{channel,head,general}_delta_step   all of these for one token of every sequence in one launch
 //
@@ -20,7 +20,7 @@
 // starts from a zero state whatever its slot holds: slots are handed on without being cleared,
 // and nothing has to be launched when a request is admitted.  A negative slot marks padding.
 //
-// Rule kernel: a CTA owns 32 value columns of one head of one sequence.  A lane holds D/8 rows x 2
+// General rule kernel: a CTA owns 32 value columns of one head of one sequence.  A lane holds D/8 rows x 2
 // columns of S in registers as row pairs (packed FP32 instructions), so the two D-long reductions
 // of a token are short chains and three shuffles; the read-out's is folded beside the next token's
 // first one.  A token depends on the one before through one reduction and one update: that chain
@@ -453,9 +453,8 @@ constexpr int kRuleBufs = 4;                         // chunks of vectors in sha
 struct RuleArgs {
   const float *q, *k, *v;         // [rows, Hk, D] x 2, [rows, H, V]
   const float* g;                 // decay [rows, H, D]
-  const float* n;                 // general: removal direction [rows, H, D]
-  const float* p;                 // general: removal rate * direction [rows, H, D]
-  const float* beta;              // channel: [rows, H]
+  const float* n;                 // removal direction [rows, H, D]
+  const float* p;                 // removal rate * direction [rows, H, D]
   float* state;                   // [slots, H, D, V]
   float* out;                     // [rows, H, V]
   const int *cu, *slots, *pos;
@@ -478,11 +477,10 @@ __device__ __forceinline__ void cp_async(float* dst, const float* src) {
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-// A token in shared memory: kVecs vectors of DP floats (g, k, q and, general, n, p), then 32
-// columns of v and beta.
-template <int DP, bool GENERAL>
+// A token in shared memory: kVecs vectors of DP floats (g, k, q, n, p), then 32 columns of v.
+template <int DP>
 struct Stage {
-  static constexpr int kVecs = GENERAL ? 5 : 3;
+  static constexpr int kVecs = 5;
   static constexpr int kToken = kVecs * DP + kCols + 4;
   static constexpr int kChunk = 8;                    // tokens per chunk
   static constexpr int kFloats = kChunk * kToken;
@@ -491,22 +489,19 @@ struct Stage {
 // Asynchronous copies of tokens' vectors by the copying threads.  Widths that are multiples of
 // four move as 16-byte pieces: a thread owns the same pieces of every token and only advances its
 // pointers (address arithmetic per piece would cost as much as the recurrence).
-template <int DP, bool GENERAL>
+template <int DP>
 struct Copier {
-  using St = Stage<DP, GENERAL>;
+  using St = Stage<DP>;
   static constexpr int kQ = DP / 4;
   static constexpr int kPieces = St::kVecs * kQ + kCols / 4;
   static constexpr int kMine = (kPieces + kRuleCopy - 1) / kRuleCopy;
   const float* src[kMine];
   int step[kMine], dst[kMine];          // floats per token, place in the token (-1: nothing)
-  const float* beta;
-  int tid, heads;
+  int tid;
   bool quad;
   __device__ __forceinline__ void init(const RuleArgs& a, int tid_, long long row0, int h, int hk, int col0) {
     tid = tid_;
-    heads = a.H;
     quad = (a.V & 3) == 0 && (a.D & 3) == 0;
-    beta = GENERAL ? nullptr : a.beta + row0 * a.H + h;
 #pragma unroll
     for (int i = 0; i < kMine; ++i) {
       const int e = tid + i * kRuleCopy, vec = e / kQ, d = (e - vec * kQ) * 4;
@@ -541,10 +536,6 @@ struct Copier {
             cp_async<16>(buf + dst[i], src[i]);
             src[i] += step[i];
           }
-        if (!GENERAL && tid == 0) {
-          cp_async<4>(buf + St::kVecs * DP + kCols, beta);
-          beta += heads;
-        }
       }
     } else {
       for (int t = 0; t < n; ++t, buf += St::kToken) {
@@ -557,16 +548,15 @@ struct Copier {
         }
         for (int c = tid; c < kCols && col0 + c < a.V; c += kRuleCopy)
           cp_async<4>(buf + St::kVecs * DP + c, a.v + (row * a.H + h) * a.V + col0 + c);
-        if (!GENERAL && tid == 0) cp_async<4>(buf + St::kVecs * DP + kCols, a.beta + row * a.H + h);
       }
     }
   }
 };
 
-template <int DP, bool GENERAL>
-__global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) vector_delta_kernel(const RuleArgs a) {
+template <int DP>
+__global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) general_delta_kernel(const RuleArgs a) {
   US_PDL_PROLOGUE();
-  using St = Stage<DP, GENERAL>;
+  using St = Stage<DP>;
   constexpr int NG = DP / 32;                         // groups of four rows per lane
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -588,7 +578,7 @@ __global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) vector_delta_k
     __syncthreads();
   }
   if (tid >= kRuleCompute) {                          // the copying threads stay one chunk ahead
-    Copier<DP, GENERAL> cp;
+    Copier<DP> cp;
     cp.init(a, tid - kRuleCompute, start, h, hk, col0);
     const int chunks = (T + St::kChunk - 1) / St::kChunk;
     auto fetch = [&](int r) {                         // (an empty group past the end)
@@ -656,18 +646,7 @@ __global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) vector_delta_k
       for (int j = 0; j < NG; ++j) {
         const int r0 = (j * 8 + kq) * 4;
         f2 m[2];
-        if (GENERAL) {
-          lds_vec(m, base + 3 * DP + r0);
-        } else {
-          f2 g[2];
-          lds_vec(m, base + DP + r0);
-          lds_vec(g, base + r0);
-#pragma unroll
-          for (int e = 0; e < 2; ++e)
-#pragma unroll
-            for (int c = 0; c < 2; ++c)     // the key sees the decayed state
-              S[j * 2 + e][c] = mul2(S[j * 2 + e][c], g[e]);
-        }
+        lds_vec(m, base + 3 * DP + r0);
 #pragma unroll
         for (int e = 0; e < 2; ++e)
 #pragma unroll
@@ -682,18 +661,10 @@ __global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) vector_delta_k
         op += ostep;
       }
       pending = true;
-      float c = seen;                               // general: n^T S of this lane's column
-      if (!GENERAL) c = vs[kCols] * (vs[cb + (up ? 1 : 0)] - seen);
-      const float other = __shfl_xor_sync(0xffffffffu, c, 4);
-      const float u0 = up ? other : c, u1 = up ? c : other;
-      f2 uu[2], vv[2];
-      if (GENERAL) {
-        const float2 v2 = *reinterpret_cast<const float2*>(vs + cb);
-        uu[0] = pack2(-u0, -u0); uu[1] = pack2(-u1, -u1);
-        vv[0] = pack2(v2.x, v2.x); vv[1] = pack2(v2.y, v2.y);
-      } else {
-        uu[0] = pack2(u0, u0); uu[1] = pack2(u1, u1);
-      }
+      const float other = __shfl_xor_sync(0xffffffffu, seen, 4);     // n^T S of this lane's column
+      const float u0 = up ? other : seen, u1 = up ? seen : other;
+      const float2 v2 = *reinterpret_cast<const float2*>(vs + cb);
+      const f2 uu[2] = {pack2(-u0, -u0), pack2(-u1, -u1)}, vv[2] = {pack2(v2.x, v2.x), pack2(v2.y, v2.y)};
       f2 oo[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
 #pragma unroll
       for (int j = 0; j < NG; ++j) {
@@ -701,17 +672,14 @@ __global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) vector_delta_k
         f2 k[2], q[2], g[2], p[2];
         lds_vec(k, base + DP + r0);
         lds_vec(q, base + 2 * DP + r0);
-        if (GENERAL) {
-          lds_vec(g, base + r0);
-          lds_vec(p, base + 4 * DP + r0);
-        }
+        lds_vec(g, base + r0);
+        lds_vec(p, base + 4 * DP + r0);
 #pragma unroll
         for (int e = 0; e < 2; ++e)
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             f2& x = S[j * 2 + e][c];
-            if (GENERAL) x = fma2(k[e], vv[c], fma2(p[e], uu[c], mul2(g[e], x)));
-            else x = fma2(k[e], uu[c], x);
+            x = fma2(k[e], vv[c], fma2(p[e], uu[c], mul2(g[e], x)));
             oo[c][e] = fma2(x, q[e], oo[c][e]);
           }
       }
@@ -1018,9 +986,9 @@ int step_impl(const StepArgs& a, int B, cudaStream_t stream) {
   return launch_step<64, RULE>(a, B, stream);
 }
 
-template <int DP, bool GENERAL>
+template <int DP>
 int launch_rule(const RuleArgs& a, int B, cudaStream_t stream) {
-  constexpr size_t need = kRuleBufs * Stage<DP, GENERAL>::kFloats * sizeof(float);
+  constexpr size_t need = kRuleBufs * Stage<DP>::kFloats * sizeof(float);
   constexpr size_t most = 227 * 1024;                 // shared memory of an SM's CTAs
   static bool configured = false;
   static int sms = 0;
@@ -1028,18 +996,18 @@ int launch_rule(const RuleArgs& a, int B, cudaStream_t stream) {
     int dev = 0;
     US_CUDA_CHECK(cudaGetDevice(&dev));
     US_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    US_CUDA_CHECK(cudaFuncSetAttribute(vector_delta_kernel<DP, GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    US_CUDA_CHECK(cudaFuncSetAttribute(general_delta_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)most));
     configured = true;
   }
   // CTAs that are launched while the kernel before still runs are packed where it leaves room, and the longest-running
-  // SM sets the time: no SM takes more than its share of them (two sequences of 4050 tokens, 32 heads of 128 x 128: 2.54 ->
-  // 2.30 ms behind a preparation that ends late).
+  // SM sets the time: no SM takes more than its share of them (two sequences of 4050 tokens, 32 heads of 64 x 64: 1.69 ->
+  // 1.17 ms behind a preparation that ends late).
   const dim3 grid((a.V + kCols - 1) / kCols, a.H, B);
   const size_t share = ((size_t)grid.x * grid.y * grid.z + sms - 1) / sms;
   size_t smem = most / (share + 1) + 1024;
   if (smem < need || share > 4) smem = need;
-  US_CUDA_CHECK(us::launch_pdl(vector_delta_kernel<DP, GENERAL>, grid, dim3(kRuleThreads), smem, stream, a));
+  US_CUDA_CHECK(us::launch_pdl(general_delta_kernel<DP>, grid, dim3(kRuleThreads), smem, stream, a));
   return US_OK;
 }
 
@@ -1146,21 +1114,19 @@ US_API int us_general_delta_prep(const void* x, long long ldx, int off_r, int of
 
 // general = 0: the channel rule (g, beta); 1: the general rule (g, n, p).  q and k heads serve
 // H / Hk value heads each; all vectors dense FP32.
-US_API int us_vector_delta_rule(int general, const float* q, const float* k, const float* v,
-                                const float* g, const float* n, const float* p, const float* beta,
-                                float* state, float* out, const int* cu, const int* slots,
-                                const int* pos, int B, int H, int Hk, int D, int V, void* stream_) {
-  US_REQUIRE(q && k && v && g && state && out && cu && slots && pos && B >= 1 && B <= 65535);
-  US_REQUIRE(general ? (n && p) : (beta != nullptr));
+US_API int us_general_delta_rule(const float* q, const float* k, const float* v, const float* g, const float* n,
+                                 const float* p, float* state, float* out, const int* cu, const int* slots,
+                                 const int* pos, int B, int H, int Hk, int D, int V, void* stream_) {
+  US_REQUIRE(q && k && v && g && n && p && state && out && cu && slots && pos && B >= 1 && B <= 65535);
   US_REQUIRE(H >= 1 && Hk >= 1 && H % Hk == 0 && H <= 65535 && D >= 1 && V >= 1);
   US_REQUIRE((D & 3) || (V & 3) || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)g | (uintptr_t)n |
                (uintptr_t)p | (uintptr_t)state) % 16) == 0);
-  RuleArgs a{q, k, v, g, n, p, beta, state, out, cu, slots, pos, H, Hk, D, V};
+  RuleArgs a{q, k, v, g, n, p, state, out, cu, slots, pos, H, Hk, D, V};
   cudaStream_t stream = (cudaStream_t)stream_;
-#define US_VD(DP) \
-  if (D <= DP) return general ? launch_rule<DP, true>(a, B, stream) : launch_rule<DP, false>(a, B, stream);
-  US_VD(32) US_VD(64) US_VD(128) US_VD(256)
-#undef US_VD
+  if (D <= 32) return launch_rule<32>(a, B, stream);
+  if (D <= 64) return launch_rule<64>(a, B, stream);
+  if (D <= 128) return launch_rule<128>(a, B, stream);
+  if (D <= 256) return launch_rule<256>(a, B, stream);
   return US_ERR_UNSUPPORTED;
 }
 

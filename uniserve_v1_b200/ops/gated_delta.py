@@ -135,7 +135,7 @@ def mixer_rows(x, offs, conv_w, conv, A, dt_bias, state, cu, slots, Hk: int, Hv:
     f = dict(dtype=torch.float32, device=x.device)
     q, k, v = torch.empty(T, Hk, Dk, **f), torch.empty(T, Hk, Dk, **f), torch.empty(T, Hv, Dv, **f)
     g, beta, out = torch.empty(T, Hv, **f), torch.empty(T, Hv, **f), torch.empty(T, Hv, Dv, **f)
-    coef = torch.empty(N.kernels().us_head_delta_coef_floats(T, B, Hv), **f)
+    coef = torch.empty(N.kernels().us_delta_coef_floats(T, B, Hv), **f)
     for t in (conv_w, conv, A, dt_bias, state):
         assert t.is_contiguous()
     assert conv_w.dtype == A.dtype == dt_bias.dtype == state.dtype == torch.float32 and conv.dtype == x.dtype

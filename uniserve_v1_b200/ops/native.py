@@ -46,7 +46,7 @@ _SIGNATURES = {
     "us_channel_delta_prep": (I, [P, L, I, I, I, I, P, P, P, P, L, P, P, P, P, P, P, P, P, P, P, P,
                                   I, I, I, I, I, I, I, I, I, P]),
     "us_general_delta_prep": (I, [P, L, I, I, I, I, P, L, P, P, P, I, I, I, F, I, P]),
-    "us_vector_delta_rule": (I, [I, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]),
+    "us_general_delta_rule": (I, [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]),
     "us_channel_delta_step": (I, [P, L, I, I, I, I, P, P, P, P, L, P, P, P, P, P, I, P, L, P, L, P, P,
                                   I, I, I, I, I, I, F, I, I, P]),
     "us_general_delta_step": (I, [P, L, I, I, I, I, P, L, P, P, P, P, I, P, L, P, L, P, P, I, I, I, F,
@@ -54,8 +54,9 @@ _SIGNATURES = {
     "us_head_delta_prep": (I, [P, L, I, I, I, I, I, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I,
                                I, I, I, I, I, P]),
     "us_window_delta_prep": (I, [P, L, I, I, I, I, I, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P]),
-    "us_head_delta_coef_floats": (L, [I, I, I]),
+    "us_delta_coef_floats": (L, [I, I, I]),
     "us_head_delta_rule": (I, [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P]),
+    "us_channel_delta_rule": (I, [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P]),
     "us_head_delta_step": (I, [P, L, I, I, I, I, I, P, P, P, P, P, P, P, P, I, P, L, P, L, P, P, I, I, I,
                                I, I, I, F, I, I, I, P]),
     "us_head_norm_gate": (I, [P, P, I, P, L, P, L, I, I, I, F, I, I, I, P]),
