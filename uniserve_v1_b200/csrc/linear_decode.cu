@@ -76,7 +76,13 @@ __device__ __forceinline__ float clamped_glu(float u, float g, float limit, floa
   return (u + 1.f) * (g / (1.f + __expf(-alpha * g)));
 }
 
-enum Form : int { kPlain = 0, kAct = 1, kClamped = 2 };
+enum Form : int { kPlain = 0, kAct = 1, kClamped = 2, kSilu = 3 };
+
+// Row tiles of a grouped launch (blockIdx.z): the experts that a few tokens chose.
+struct Group {
+  const int *group, *row0, *rows, *count;     // weight block, first row and rows of every tile; how many tiles
+  long long stride;                           // elements of a weight block
+};
 
 struct Glu {
   int second;             // weight row of the first feature of the second half
@@ -86,17 +92,26 @@ struct Glu {
 };
 
 // MT = 16-row tiles of the activation (rows <= 16 * MT).
-template <int MT, int FORM>
+template <int MT, int FORM, bool GROUPED = false>
 __global__ void __launch_bounds__(256)
 linear_decode_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ X,
                      void* __restrict__ out, const void* __restrict__ bias, int rows, int M, int K,
                      long long ldw, long long ldx, long long ldo, int out_f32, int bias_f32,
-                     int ksplit, const Glu glu) {
-  constexpr bool ACT = FORM == kAct, GATED = FORM == kClamped;
+                     int ksplit, const Glu glu, const Group grp) {
+  constexpr bool ACT = FORM == kAct, GATED = FORM == kClamped || FORM == kSilu;
   constexpr int kOut = GATED ? kFeat / 2 : kFeat;       // output features per CTA
   // Weights are never written by a kernel: the first loads go out before the wait on the
   // kernels that produce the activation.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (GROUPED) {                                        // which weights they are is known only then
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if ((int)blockIdx.z >= *grp.count) return;
+    const long long row0 = grp.row0[blockIdx.z];
+    W += grp.group[blockIdx.z] * grp.stride;
+    X += row0 * ldx;
+    rows = grp.rows[blockIdx.z];
+    out = reinterpret_cast<__nv_bfloat16*>(out) + row0 * ldo;
+  }
   // activation tiles [kStages][rows][pieces] (a cp.async ring, kStages - 1 tiles in flight:
   // the tiles come from L2, a tile's arithmetic is far shorter than its latency); the
   // K-slice partial sums [slice][group][row][8 + 1] reuse the memory after the loop
@@ -128,7 +143,7 @@ linear_decode_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* _
   };
 #pragma unroll
   for (int a = 0; a < kAhead; ++a) load_w(a, wreg[a]);
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!GROUPED) asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // activation tile of iteration it: rows x 256 k, 16-byte pieces by all threads
   auto load_x = [&](int it, int buf) {
@@ -217,7 +232,7 @@ linear_decode_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* _
         const int col = blockIdx.x * kOut + f;
         if (r >= rows || col >= M) continue;
         float v = whole(r, f);
-        if (GATED) v = clamped_glu(v, whole(r, f + 8), glu.limit, glu.alpha);
+        if (FORM == kClamped) v = clamped_glu(v, whole(r, f + 8), glu.limit, glu.alpha);
         if (bias)
           v += bias_f32 ? reinterpret_cast<const float*>(bias)[col]
                         : us::bf2f(reinterpret_cast<const __nv_bfloat16*>(bias)[col]);
@@ -242,7 +257,11 @@ linear_decode_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* _
     const int col = blockIdx.x * kOut + f;
     if (r >= rows || col >= M) continue;
     float v = sliced(r, f);
-    if (GATED) v = clamped_glu(v, sliced(r, f + 8), glu.limit, glu.alpha);
+    if (FORM == kClamped) v = clamped_glu(v, sliced(r, f + 8), glu.limit, glu.alpha);
+    if (FORM == kSilu) {
+      const float g = sliced(r, f + 8);
+      v *= g / (1.f + __expf(-g));
+    }
     if (bias)
       v += bias_f32 ? reinterpret_cast<const float*>(bias)[col]
                     : us::bf2f(reinterpret_cast<const __nv_bfloat16*>(bias)[col]);
@@ -307,7 +326,7 @@ int run(int form, const void* W, const void* X, void* out, const void* bias, int
     cfg.attrs = attr;
     cfg.numAttrs = ksplit > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, w, x, out, bias, rows, M, K, ldw, ldx, ldo, out_f32,
-                              bias_f32, ksplit, glu);
+                              bias_f32, ksplit, glu, Group{});
   };
   // kStages buffers x (16 MT) rows x 512 bytes
 #define US_LD(MT)                                                                                \
@@ -342,4 +361,23 @@ US_API int us_linear_decode_clamped(const void* W, const void* X, void* out, int
   US_REQUIRE(W && X && out && rows >= 1 && I >= 1 && K >= 1);
   return run(kClamped, W, X, out, nullptr, rows, I, K, ldw, ldx, ldo, 0, 0, Glu{I, limit, alpha, 0, 0.f, 0.f},
              (cudaStream_t)stream_);
+}
+
+// Grouped: for every tile of at most 16 rows, out = X W_group^T, or with `silu` first * silu(second) (W_group [2 M, K]
+// stacks their rows).  W [groups, (2) M, K] and X dense, out [., M]; K a multiple of 256.  For the experts of a few
+// tokens: a CTA per 16 (gated 8) features has ten times the loads in flight of one per 128, which is what a stream of
+// few weights lacks.
+US_API int us_linear_decode_grouped(const void* W, const void* X, void* out, int M, int K, int silu,
+                                    const int* tile_group, const int* tile_row0, const int* tile_rows,
+                                    const int* num_tiles, int max_tiles, void* stream_) {
+  US_REQUIRE(W && X && out && M >= 1 && K >= 1 && tile_group && tile_row0 && tile_rows && num_tiles);
+  US_REQUIRE(max_tiles >= 1 && max_tiles <= 65535);
+  if ((K % kIterK) != 0 || ((uintptr_t)W % 16) != 0 || ((uintptr_t)X % 16) != 0) return US_ERR_UNSUPPORTED;
+  const Group grp{tile_group, tile_row0, tile_rows, num_tiles, (long long)(silu ? 2 : 1) * M * K};
+  const dim3 grid(us::ceil_div(M, silu ? kFeat / 2 : kFeat), 1, max_tiles);
+  auto kernel = silu ? linear_decode_kernel<1, kSilu, true> : linear_decode_kernel<1, kPlain, true>;
+  US_CUDA_CHECK(us::launch_pdl(kernel, grid, dim3(256), kStages * 8192, (cudaStream_t)stream_, (const __nv_bfloat16*)W,
+                               (const __nv_bfloat16*)X, out, (const void*)nullptr, 16, M, K, (long long)K, (long long)K,
+                               (long long)M, 0, 0, 1, Glu{M, 0.f, 0.f, 0, 0.f, 0.f}, grp));
+  return US_OK;
 }

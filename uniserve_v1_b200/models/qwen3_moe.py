@@ -491,7 +491,7 @@ class Qwen3MoeModel:
             if ws is None:
                 ws = F.MoeWorkspace.create(T, cfg.num_experts_per_tok, self.E_local,
                                            cfg.hidden_size, cfg.moe_intermediate_size, x.device,
-                                           E_total=cfg.num_experts)
+                                           E_total=cfg.num_experts, fp8=lw.fp8 is not None)
                 self._moe_ws[key] = ws
         # distributed weight data parallelism: every expert runs here, on weights read from the
         # peers' resident shards; tokens stay, so nothing is reduced across ranks
@@ -522,7 +522,7 @@ class Qwen3MoeModel:
             if ws is not None and ws.block_n > 64:
                 ws = self._moe_ws[key] = F.MoeWorkspace.create(
                     T, cfg.num_experts_per_tok, self.E_local, cfg.hidden_size,
-                    cfg.moe_intermediate_size, x.device, block_n=64)
+                    cfg.moe_intermediate_size, x.device, fp8=True)
             out = moe_experts_fp8(x, ids, weights, lw.fp8, e_lo=self.e_lo, ws=ws)
         else:
             later = defer and small and FUSED_UNPERMUTE and (fc is not None or not reduce)

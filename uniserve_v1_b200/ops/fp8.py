@@ -162,7 +162,7 @@ def moe_experts_fp8(x, ids, weights, ex: Fp8Experts, e_lo=0, act="silu", ws=None
     E, I2, _ = ex.w13.shape
     I_ = I2 // 2
     if ws is None:
-        ws = MoeWorkspace.create(T, top_k, E, H, I_, x.device)
+        ws = MoeWorkspace.create(T, top_k, E, H, I_, x.device, fp8=True)
     if ws.block_n > 64:
         raise ValueError("the gated FP8 GEMM serves row tiles of at most 64")
     R_ = T * top_k

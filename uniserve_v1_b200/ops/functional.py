@@ -437,7 +437,22 @@ def topk_softmax(logits, top_k, renorm=True, live=None, expert_map=None, load=No
 
 # rows per local expert from which the grouped expert GEMMs take 256-row tiles on the CTA-pair
 # kernel (US_MOE_PAIR_ROWS; a huge value keeps the single-CTA kernel)
-MOE_PAIR_MIN_ROWS = int(_os.environ.get("US_MOE_PAIR_ROWS", "64"))
+MOE_PAIR_MIN_ROWS = int(_os.environ.get("US_MOE_PAIR_ROWS", "96"))
+
+
+def _tile_rows(per: float, gated: bool = True, fp8: bool = False) -> int:
+    """Rows per tile for ``per`` routes to an expert on average (single-CTA kernels).  A tile streams its expert's
+    weights, so two tiles of an expert cost up to twice one; a wider one multiplies more empty rows and holds fewer
+    stages.  Measured at 128 experts of 2048 x 768 and 4096 x 1536 and 64 of 2048 x 768 (us of a whole layer, rows per
+    tile 16 / 32 / 64, CTA pairs of 256): 13 routes 229 / 219 / 252 / 431, 25 routes 273 / 233 / 285 / 435, 56 routes 425 / 316 /
+    343 / 452, 75 routes - / 370 / 456 / 449, 113 routes - / 474 / 551 / 456; below 4 routes 16 and 32 change places within 3 %.
+    FP8: 6 routes 164 / 169, 16 routes 607 / 532 / 780, 56 routes 461 / 385 / 597.  Ungated (64 experts of 2048 x 1024): 4 routes
+    95 / 96 / 96, 16 routes 109 / 104 / 104, 32 routes 139 / 127 / 115, 64 routes 185 / 155 / 146 / 161, 94 routes 249 / 194 / 167 / 163."""
+    if fp8:
+        return 16 if per <= 10 else 32
+    if gated:
+        return 16 if per < 4 else 32 if per < 96 else 128
+    return 16 if per < 12 else 32 if per < 24 else 64 if per < 96 else 128
 
 
 @dataclass
@@ -459,15 +474,14 @@ class MoeWorkspace:
     live_tiles: int = 0                   # expected number of non-empty row tiles
 
     @staticmethod
-    def create(T, top_k, E_local, H, I, device, block_n=None, E_total=None):
+    def create(T, top_k, E_local, H, I, device, block_n=None, E_total=None, fp8=False):
         """``E_total``: experts of the whole model when this rank holds only ``E_local`` of
         them (the routes then spread over all ranks; sizes the expected live tiles)."""
         R_ = T * top_k
         if block_n is None:
-            avg = max(1, R_ // max(1, E_local))
-            block_n = 16 if avg <= 16 else 32 if avg <= 32 else 64 if avg <= 64 else 128
+            block_n = _tile_rows(R_ / max(1, E_local), fp8=fp8)
             # prefill-size batches (a few hundred rows per expert): 256-row tiles on CTA pairs
-            if R_ // max(1, E_total or E_local) >= MOE_PAIR_MIN_ROWS:
+            if not fp8 and R_ // max(1, E_total or E_local) >= MOE_PAIR_MIN_ROWS:
                 block_n = 256
         max_tiles = min(R_, E_local) + R_ // block_n + 1
         i32 = dict(dtype=torch.int32, device=device)
@@ -543,6 +557,12 @@ def unpermute_add_rmsnorm(y_perm, perm, weights, residual, w, eps=1e-6):
     return y, residual
 
 
+# Routed weights (of one product's half, elements) up to which a few tokens' experts take the weight-streaming kernel:
+# a row tile of 128 features per CTA leaves most SMs idle.  Layers of one token measured 45 -> 37 us (8 of 128 experts of
+# 2048 x 768) and 40 -> 24 us (4 of 64); with 16 experts of that size 53 -> 59, with 8 of 4096 x 1536 83 -> 112.
+MOE_STREAM_WEIGHTS = int(_os.environ.get("US_MOE_STREAM", str(16 << 20)))
+
+
 def moe_experts(x, ids, weights, w13, w2, e_lo=0, act="silu", stepwise=False, ws=None, out=None,
                 presorted=False, pregathered=False, defer_unpermute=False):
     """Routed experts: sort routes by local expert, gather rows, grouped FC1 with
@@ -571,6 +591,12 @@ def moe_experts(x, ids, weights, w13, w2, e_lo=0, act="silu", stepwise=False, ws
         N.call("us_moe_gather", N.ptr(x), N.ptr(ws.sorted_route), N.ptr(total), R_, top_k, H,
                N.ptr(ws.xp), st)
     code = _ACT["silu_stepwise" if (act == "silu" and stepwise) else act]
+    if R_ * H * I_ <= MOE_STREAM_WEIGHTS and code == 0 and ws.block_n == 16 and H % 256 == 0 and I_ % 256 == 0 and \
+            all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (w13, w2)):
+        tiles = (N.ptr(ws.tile_group), N.ptr(ws.tile_row0), N.ptr(ws.tile_rows), N.ptr(ws.num_tiles), ws.max_tiles)
+        N.call("us_linear_decode_grouped", N.ptr(w13), N.ptr(ws.xp), N.ptr(ws.h), I_, H, 1, *tiles, st)
+        N.call("us_linear_decode_grouped", N.ptr(w2), N.ptr(ws.h), N.ptr(ws.y), H, I_, 0, *tiles, st)
+        return _unpermuted(ws, weights, out, T, top_k, H, defer_unpermute, x.device, st)
     # FC1: [R, H] x [E, 2I, H] -> [R, I] with first * act(gate)
     live = ws.live_tiles
     if live:
@@ -584,10 +610,14 @@ def moe_experts(x, ids, weights, w13, w2, e_lo=0, act="silu", stepwise=False, ws
     N.call("us_gemm_wx", N.ptr(w2), N.ptr(ws.h), N.ptr(ws.y), E, H, H, I_, R_, I_, I_, H, 0, 0, 0,
            0, None, 0, None, None, N.ptr(ws.tile_group), N.ptr(ws.tile_row0), N.ptr(ws.tile_rows),
            N.ptr(ws.num_tiles), ws.max_tiles, ws.block_n, st)
-    if defer_unpermute:
+    return _unpermuted(ws, weights, out, T, top_k, H, defer_unpermute, x.device, st)
+
+
+def _unpermuted(ws, weights, out, T, top_k, H, defer, device, st):
+    if defer:
         return ws.y, ws.perm_of_route.view(T, top_k)
     if out is None:
-        out = torch.empty(T, H, dtype=BF16, device=x.device)
+        out = torch.empty(T, H, dtype=BF16, device=device)
     N.call("us_moe_unpermute", N.ptr(ws.y), N.ptr(ws.perm_of_route), N.ptr(weights), T, top_k, H,
            N.ptr(out), st)
     return out
@@ -616,20 +646,19 @@ class Routes:
                 N.ptr(self.num_tiles), self.max_tiles)
 
 
-def _route_tiles(R_, E, E_total):
+def _route_tiles(R_, E, E_total, gated=True):
     """(rows per tile, most tiles, expected live tiles) of R_ routes over E_total experts, E of them here."""
-    avg = max(1, R_ // E_total)
-    block_n = 16 if avg <= 16 else 32 if avg <= 32 else 64 if avg <= 64 else 128
-    if avg >= MOE_PAIR_MIN_ROWS:
+    block_n = _tile_rows(R_ / E_total, gated)
+    if R_ // E_total >= MOE_PAIR_MIN_ROWS:
         block_n = 256
     return block_n, min(R_, E) + R_ // block_n + 1, MoeWorkspace._expected_tiles(R_, E, E_total, block_n)
 
 
-def _route(logits, top, E, E_all, x, gather, pick):
+def _route(logits, top, E, E_all, x, gather, pick, gated):
     """Routes of ``logits``: ``gather(ids, weights, sort, xp)`` in one launch up to 512 rows of ``x``, above
-    ``pick(ids, weights)`` and a sort."""
+    ``pick(ids, weights)`` and a sort.  ``gated``: whether the experts are (sizes their row tiles)."""
     T, dev, R_ = logits.shape[0], logits.device, logits.shape[0] * top
-    block_n, max_tiles, live = _route_tiles(R_, E, E_all)
+    block_n, max_tiles, live = _route_tiles(R_, E, E_all, gated)
     buf = torch.empty(3 * R_ + E + 1 + 3 * max_tiles + 1, dtype=torch.int32, device=dev)
     ids, srt, perm, offs, tg, t0, tr, nt = buf.split([R_, R_, R_, E + 1, max_tiles, max_tiles, max_tiles, 1])
     weights = torch.empty(T, top, dtype=torch.float32, device=dev)
@@ -660,7 +689,7 @@ def grouped_routes(logits, E, top, groups, scale, x, sync):
         lambda ids, weights, sort, rows: N.call("us_grouped_route_sort_gather", N.ptr(logits), ld, ids, weights, T, E,
                                                 top, per, keep, scale, *sort, *rows, N.ptr(sync), st),
         lambda ids, weights: N.call("us_grouped_topk", N.ptr(logits), ld, ids, weights, T, E, top, per, keep, scale,
-                                    st))
+                                    st), gated=False)
 
 
 def scored_routes(logits, correction, top, E, x, sync):
@@ -678,7 +707,7 @@ def scored_routes(logits, correction, top, E, x, sync):
         lambda ids, weights, sort, rows: N.call("us_route_sort_gather", N.ptr(logits), ids, weights, T, E_all, top, 1,
                                                 None, 0, E, *sort, *rows, N.ptr(sync), N.ptr(correction), st),
         lambda ids, weights: N.call("us_topk_softmax", N.ptr(logits), ids, weights, T, E_all, top, 1, None, None, None,
-                                    N.ptr(correction), st))
+                                    N.ptr(correction), st), gated=True)
 
 
 def table_routes(tokens, tables, E):
@@ -690,7 +719,7 @@ def table_routes(tokens, tables, E):
     if not _cuda(tokens):
         return [R.table_routes(tokens, tables[i]) for i in range(Ln)]
     R_ = T * top
-    block_n, max_tiles, live = _route_tiles(R_, E, E)
+    block_n, max_tiles, live = _route_tiles(R_, E, E, False)
     widths = (R_, R_, R_, E + 1, max_tiles, max_tiles, max_tiles, 1)
     buf = torch.empty(Ln * sum(widths), dtype=torch.int32, device=tokens.device)
     parts, off = [], 0

@@ -41,6 +41,7 @@ _SIGNATURES = {
     "us_gemm_wx_hint": (I, [I]),
     "us_linear_decode": (I, [P, P, P, P, I, I, I, L, L, L, I, I, I, F, F, P]),
     "us_gemm_wx_act": (I, [P, P, P, I, I, I, I, I, L, L, L, I, F, F, P, P, P, P, I, I, P]),
+    "us_linear_decode_grouped": (I, [P, P, P, I, I, I, P, P, P, P, I, P]),
     "us_linear_decode_clamped": (I, [P, P, P, I, I, I, L, L, L, F, F, P]),
     "us_gemm_f32": (I, [P, P, P, I, I, I, I, I, L, L, L, I, F, F, P, P, P, P, P, I, P]),
     "us_channel_delta_prep": (I, [P, L, I, I, I, I, P, P, P, P, L, P, P, P, P, P, P, P, P, P, P, P,
