@@ -95,16 +95,33 @@ kv_write_scaled_kernel(const __nv_bfloat16* __restrict__ k_src, const __nv_bfloa
 // Packed context rows of a batch: sequence s contributes rows [0, cu[s + 1] - cu[s]) of its
 // pages to out rows [out_cu[s], ...) (out_cu = cu unless the caller leaves room behind each
 // sequence's cached rows for its new ones).  grid (row tiles of 8, 2 planes); a warp moves
-// one row.
+// one row.  Rows past the cached ones, if asked for, are the call's new keys and values on their way to their places
+// behind each sequence's cached rows (two scatters of their own before: 3.6 us and two launches more a layer).
+struct NewRows {
+  const __nv_bfloat16 *k, *v;       // [count, ld]
+  const long long* dst;             // out row of each
+  long long ld;
+  int count, cached;                // rows of the grid before them
+};
+
 __global__ void __launch_bounds__(256)
 kv_gather_kernel(const void* __restrict__ k_cache, const void* __restrict__ v_cache,
                  const float* __restrict__ k_scale, const float* __restrict__ v_scale,
                  const int* __restrict__ page_table, int max_pages, const int* __restrict__ cu,
                  const int* __restrict__ out_cu, int B, int page_size, int row_elems, __nv_bfloat16* __restrict__ k_out,
-                 __nv_bfloat16* __restrict__ v_out, long long ldo, int fp8) {
+                 __nv_bfloat16* __restrict__ v_out, long long ldo, int fp8, const NewRows nw) {
   US_PDL_PROLOGUE();
   const int total = cu[B];
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= nw.cached) {
+    const int j = r - nw.cached;
+    if (j >= nw.count) return;
+    const __nv_bfloat16* src = (blockIdx.y == 1 ? nw.v : nw.k) + j * nw.ld;
+    __nv_bfloat16* dst = (blockIdx.y == 1 ? v_out : k_out) + nw.dst[j] * ldo;
+    for (int e = lane * 8; e < row_elems; e += 256)
+      *reinterpret_cast<uint4*>(dst + e) = *reinterpret_cast<const uint4*>(src + e);
+    return;
+  }
   if (r >= total) return;
   int lo = 0, hi = B - 1;                       // sequence of packed row r
   while (lo < hi) {
@@ -160,13 +177,17 @@ US_API int us_kv_write_scaled(const void* k_src, const void* v_src, long long ld
 US_API int us_kv_gather(const void* k_cache, const void* v_cache, const float* k_scale,
                         const float* v_scale, const int* page_table, int max_pages, const int* cu,
                         const int* out_cu, int B, int total_rows, int page_size, int heads, int head_dim, void* k_out,
-                        void* v_out, long long ldo, int fp8, void* stream_) {
+                        void* v_out, long long ldo, int fp8, const void* k_new, const void* v_new, long long ldn,
+                        const long long* new_dst, int new_rows, void* stream_) {
   US_REQUIRE(k_cache && v_cache && page_table && cu && k_out && v_out && B >= 1);
   US_REQUIRE(((heads * head_dim) % 8) == 0 && (ldo % 8) == 0 && (!fp8 || (k_scale && v_scale)));
-  if (total_rows == 0) return US_OK;
-  US_CUDA_CHECK(us::launch_pdl(kv_gather_kernel, dim3((total_rows + 7) / 8, 2), dim3(256), 0,
+  US_REQUIRE(new_rows >= 0 && (new_rows == 0 || (k_new && v_new && new_dst && ldn % 8 == 0 &&
+             (((uintptr_t)k_new | (uintptr_t)v_new) % 16) == 0)));
+  if (total_rows + new_rows == 0) return US_OK;
+  const NewRows nw{(const __nv_bfloat16*)k_new, (const __nv_bfloat16*)v_new, new_dst, ldn, new_rows, total_rows};
+  US_CUDA_CHECK(us::launch_pdl(kv_gather_kernel, dim3((total_rows + new_rows + 7) / 8, 2), dim3(256), 0,
                                (cudaStream_t)stream_, k_cache, v_cache, k_scale, v_scale, page_table,
                                max_pages, cu, out_cu ? out_cu : cu, B, page_size, heads * head_dim,
-                               (__nv_bfloat16*)k_out, (__nv_bfloat16*)v_out, ldo, fp8));
+                               (__nv_bfloat16*)k_out, (__nv_bfloat16*)v_out, ldo, fp8, nw));
   return US_OK;
 }

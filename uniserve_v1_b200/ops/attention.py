@@ -57,18 +57,19 @@ def prefill_attention(qkv, Hq, Hkv, D, meta, kcache, vcache, scale):
     if ctx_lens is not None and any(c > 0 for c in ctx_lens):
         tables = getattr(meta, "ctx_tables", None)
         if qkv.is_cuda and tables is not None:
-            # Keys already cached sit in front of this call's keys of each sequence: one
-            # gather launch through the page table (bf16 or E4M3 pages) and one row scatter
-            # of the new keys; nothing returns to the host.
+            # Keys already cached sit in front of this call's keys of each sequence: one launch gathers
+            # them through the page table (bf16 or E4M3 pages) and puts the new ones behind; nothing
+            # returns to the host.
             from . import functional as F
             ctx_cu, new_dst, ctx_total = tables
             total = ctx_total + new_dst.shape[0]
             kb = torch.empty(total, Hkv, D, dtype=qkv.dtype, device=qkv.device)
             vb = torch.empty(total, Hkv, D, dtype=qkv.dtype, device=qkv.device)
             F.kv_gather(kcache, vcache, meta.page_table, ctx_cu, ctx_total, k_scale, v_scale,
-                        out=(kb, vb), out_cu=meta.cu_k)
-            kb.index_copy_(0, new_dst, k[:new_dst.shape[0]])
-            vb.index_copy_(0, new_dst, v[:new_dst.shape[0]])
+                        out=(kb, vb), out_cu=meta.cu_k, new=(k, v, new_dst) if D % 8 == 0 else None)
+            if D % 8:                     # heads that do not start on 16 bytes
+                kb.index_copy_(0, new_dst, k[:new_dst.shape[0]])
+                vb.index_copy_(0, new_dst, v[:new_dst.shape[0]])
             k, v = kb, vb
         else:
             page = kcache.shape[1]

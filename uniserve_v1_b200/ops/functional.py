@@ -203,12 +203,22 @@ def kv_write_scaled(k, v, slots, kcache, vcache, k_scale, v_scale):
            N.stream())
 
 
+def _new_rows(new):
+    if new is None:
+        return None, None, 0, None, 0
+    k, v, dst = new
+    assert k.dtype == v.dtype == BF16 and k.stride(0) == v.stride(0) and k.shape[0] >= dst.shape[0]
+    assert all(t.stride(2) == 1 and t.stride(1) == t.shape[2] for t in (k, v)) and dst.dtype == torch.int64
+    return N.ptr(k), N.ptr(v), k.stride(0), N.ptr(dst), dst.shape[0]
+
+
 def kv_gather(kcache, vcache, page_table, cu, total_rows, k_scale=None, v_scale=None, out=None,
-              out_cu=None):
+              out_cu=None, new=None):
     """Cached rows of a batch as packed bf16: sequence s contributes its first
     cu[s + 1] - cu[s] cached positions (through ``page_table`` [B, max_pages]) to rows
     [cu[s], cu[s + 1]) of the result ([total_rows, Hkv, D] for K and for V), or to rows
     starting at ``out_cu[s]`` of a larger ``out``.  Pages are bf16, or E4M3 with scales.
+    ``new`` = (k, v, dst): rows [n, Hkv, D] (bf16, heads dense) that go to the rows ``dst`` (int64) of ``out`` as well.
     Nothing is read back to the host."""
     pages, page, Hkv, D = kcache.shape
     B = page_table.shape[0]
@@ -219,7 +229,7 @@ def kv_gather(kcache, vcache, page_table, cu, total_rows, k_scale=None, v_scale=
     fp8 = k_scale is not None
     N.call("us_kv_gather", N.ptr(kcache), N.ptr(vcache), N.ptr(k_scale) if fp8 else None,
            N.ptr(v_scale) if fp8 else None, N.ptr(page_table), page_table.shape[1], N.ptr(cu),
-           N.ptr(out_cu) if out_cu is not None else None, B, total_rows, page, Hkv, D, N.ptr(ko), N.ptr(vo), ko.stride(0), int(fp8), N.stream(),
+           N.ptr(out_cu) if out_cu is not None else None, B, total_rows, page, Hkv, D, N.ptr(ko), N.ptr(vo), ko.stride(0), int(fp8), *_new_rows(new), N.stream(),
            launches=1)
     return ko, vo
 

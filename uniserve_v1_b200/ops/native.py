@@ -82,7 +82,7 @@ _SIGNATURES = {
     "us_head_mix_prefill": (I, [P, P, P, P, P, P, P, P, L, L, I, I, I, I, I, I, I, I, I, I, F, P]),
     "us_table_route_sort": (I, [P, P, I, I, I, I, I, I, I, P, P, P, P, P, P, P, P, P]),
     "us_kv_write_scaled": (I, [P, P, L, L, P, P, P, P, P, I, I, I, I, P]),
-    "us_kv_gather": (I, [P, P, P, P, P, I, P, P, I, I, I, I, I, P, P, L, I, P]),
+    "us_kv_gather": (I, [P, P, P, P, P, I, P, P, I, I, I, I, I, P, P, L, I, P, P, L, P, I, P]),
     "us_paged_decode_attention_fp8": (I, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I,
                                           F, L, L, P]),
     "us_causal_conv1d": (I, [P, L, P, P, P, L, P, P, I, I, I, I, I, I, P]),
