@@ -13,32 +13,41 @@
 //
 // No quotient of decays is formed: a product over a span is taken factor by factor, so nothing overflows.
 //
-// The chain from chunk to chunk is three small products.  They run on the tensor cores with FP32 operands split into
-// two TF32 parts each and three products (22 bits of a product; sums in FP32).  Token by token, or four tokens at a
-// time on the FP32 units, a chunk's sixteen tokens took sixteen or four rounds of shuffles and dependent sums.
-// mma.sync and not tcgen05: a chunk's operands come from registers (the state's accumulators are the next product's A
-// operand as they stand, its channels merely taken in another order), and a round through tensor memory costs
-// more than these products do.
+// The chain from chunk to chunk is three small products.  They run on the tensor cores with FP32 operands in three
+// bf16 parts, which hold all 24 bits, and the six products of parts that reach them (what is left out is 2^-25 of a
+// product and less).  The units round sums towards zero.  So products of leading parts are summed over sixteen
+// channels or tokens at a time, from zero, and added on the FP32 units; the leading part of every operand but the state
+// and U has only six bits, which leaves such a sum room for nearly all of its bits; the smaller products have a sum of
+// their own.  Token by token, or four tokens at a time on the FP32 units, a chunk took sixteen or four rounds of
+// shuffles and dependent sums.  mma.sync and not tcgen05: a chunk's operands come from registers (the state's
+// accumulators are the next product's A operand as they stand), and a round through tensor memory costs more than
+// these products do.
 //
-// A CTA owns 32 value columns of one head of one sequence: two tiles of sixteen columns, each two warps that share
-// the channels.  A warp holds S^T [16 columns, D / 2 channels] as accumulators.  Partial K S0 and Q S0 meet in shared
-// memory; both warps of a tile solve U.  The vectors of the next chunks are fetched into a ring in shared memory; with a
-// decay per channel they are multiplied with their decays there, a chunk ahead.  A sequence whose first packed row
-// stands at position 0 starts from a zero state whatever its slot holds; a negative slot marks padding.
+// A CTA owns 32 value columns of one head of one sequence.  Four warps carry the chain: two tiles of sixteen columns,
+// each two warps that share the channels.  Such a warp holds S^T [16 columns, D / 2 channels] as accumulators.  Partial
+// K S0 and Q S0 meet in shared memory; both warps of a tile solve U.  Four more warps do what is not on the chain: they
+// fetch the next chunk's vectors, multiply them with their decays where those are per channel, and lay their parts out
+// in shared memory, two chunks at most, and they form a chunk's outputs while the next one is under way.  A sequence
+// whose first packed row stands at position 0 starts from a zero state whatever its slot holds; a negative slot marks
+// padding.
 #include "include/us_common.cuh"
+#include "include/us_f32x2.cuh"
+#include "include/us_mma.cuh"
 
 namespace {
+
+using namespace us::f32x2;
 
 constexpr int kChunk = 16;        // tokens whose products share a state
 constexpr int kCols = 32;         // value columns per CTA
 constexpr int kSplit = 2;         // warps that share a tile's channels
 constexpr int kTiles = kCols / 16;
-constexpr int kThreads = 32 * kSplit * kTiles;
-constexpr int kBufs = 3;          // chunks in shared memory
+constexpr int kCompute = 32 * kSplit * kTiles, kFeed = 128, kThreads = kCompute + kFeed;
 constexpr int kMaxDim = 256;
 
-// Coefficients of a chunk and head: M [t][i] | W [t][i] | with a decay per head P_t | R_t16
-constexpr int kM = 0, kW = 256, kP = 512, kR = 528, kCoef = 544;
+// Coefficients of a chunk and head: M [t][i] and W [t][i] below their diagonals, as three bf16 parts each | beta_t and
+// W_tt, the diagonals | with a decay per head P_t | R_t16
+constexpr int kMat = 3 * kChunk * kChunk / 2, kDiag = 2 * kMat, kP = kDiag + 2 * kChunk, kCoef = kP + 2 * kChunk;
 
 struct DeltaRule {
   const float *q, *k, *v;         // [rows, Hk, D] x 2, [rows, H, V]
@@ -65,18 +74,65 @@ __device__ __forceinline__ bool find_chunk(const DeltaRule& a, int& s, int& star
   return false;
 }
 
-// M from L (strictly lower) and beta: column `lane` by forward substitution.
-__device__ __forceinline__ void solve_columns(const float (*low)[kChunk + 1], const float* beta, float* out, int lane) {
-  if (lane >= kChunk) return;
-  float m[kChunk];
+// x to six bits; what remains of it is the sum of two bf16
+__device__ __forceinline__ float leading(float x) {
+  return __uint_as_float((__float_as_uint(x) + 0x20000u) & 0xfffc0000u);
+}
+// (x, y) = sum of three bf16 pairs, the first of six bits each
+__device__ __forceinline__ void split(float x, float y, uint32_t (&o)[3]) {
+  const float a = leading(x), b = leading(y);
+  o[0] = us::pack_bf(a, b);
+  x -= a;
+  y -= b;
 #pragma unroll
-  for (int x = 0; x < kChunk; ++x) {
-    float sum = x == lane ? beta[x] : 0.f;
-#pragma unroll
-    for (int y = 0; y < x; ++y) sum = fmaf(-low[x][y], m[y], sum);
-    m[x] = sum;
-    out[kM + x * kChunk + lane] = sum;
+  for (int i = 1; i < 3; ++i) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+    o[i] = *reinterpret_cast<const uint32_t*>(&p);
+    x -= us::bf2f(p.x);
+    y -= us::bf2f(p.y);
   }
+}
+
+// Eight neighbours of row t of matrix 0 (M) or 1 (W), what stands below the diagonal.
+__device__ __forceinline__ void put_coefs(float* coef, int matrix, int t, int i0, const float (&x)[8]) {
+  uint32_t o[4][3];
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    split(i0 + 2 * e < t ? x[2 * e] : 0.f, i0 + 2 * e + 1 < t ? x[2 * e + 1] : 0.f, o[e]);
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+    *reinterpret_cast<uint4*>(coef + matrix * kMat + (p * kChunk * kChunk + t * kChunk + i0) / 2) =
+        make_uint4(o[0][p], o[1][p], o[2][p], o[3][p]);
+}
+
+// M from L (strictly lower) and beta, by forward substitution: a lane per column, then a lane per half a row.
+__device__ __forceinline__ void solve(float (*low)[kChunk + 1], const float* beta, float* out, int lane) {
+  float m[kChunk];
+  if (lane < kChunk) {
+#pragma unroll
+    for (int x = 0; x < kChunk; ++x) {
+      float sum = x == lane ? beta[x] : 0.f;
+#pragma unroll
+      for (int y = 0; y < x; ++y) sum = fmaf(-low[x][y], m[y], sum);
+      m[x] = sum;
+    }
+  }
+  __syncwarp();
+  if (lane < kChunk) {
+#pragma unroll
+    for (int x = 0; x < kChunk; ++x) low[x][lane] = m[x];
+    out[kDiag + lane] = beta[lane];
+  }
+  __syncwarp();
+  const int t = lane >> 1, i0 = (lane & 1) * 8;
+  float row[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) row[e] = low[t][i0 + e];
+  put_coefs(out, 0, t, i0, row);
+}
+
+__device__ __forceinline__ float dot4(const float4& x, const float4& y, float sum) {
+  return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, sum))));
 }
 
 constexpr int kGramWarps = 4, kGramPitch = 36;   // 32 channels at a time, rows apart by 4 banks
@@ -109,16 +165,27 @@ __global__ void __launch_bounds__(kGramWarps * 32) head_gram_kernel(const DeltaR
       qr[e * kGramPitch + lane] = in ? a.q[at] : 0.f;
     }
     __syncwarp();
+    float k32[8], q32[8];                            // chains of eight products, then of 32: short ones round less
 #pragma unroll
-    for (int d = 0; d < 32; d += 4) {
+    for (int e = 0; e < 8; ++e) k32[e] = q32[e] = 0.f;
+#pragma unroll
+    for (int d = 0; d < 32; d += 8) {
       const float4 kt = *reinterpret_cast<const float4*>(kr + t * kGramPitch + d);
       const float4 qt = *reinterpret_cast<const float4*>(qr + t * kGramPitch + d);
+      const float4 kt4 = *reinterpret_cast<const float4*>(kr + t * kGramPitch + d + 4);
+      const float4 qt4 = *reinterpret_cast<const float4*>(qr + t * kGramPitch + d + 4);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float4 ki = *reinterpret_cast<const float4*>(kr + (i0 + e) * kGramPitch + d);
-        kk[e] = fmaf(kt.x, ki.x, fmaf(kt.y, ki.y, fmaf(kt.z, ki.z, fmaf(kt.w, ki.w, kk[e]))));
-        qk[e] = fmaf(qt.x, ki.x, fmaf(qt.y, ki.y, fmaf(qt.z, ki.z, fmaf(qt.w, ki.w, qk[e]))));
+        const float4 ki4 = *reinterpret_cast<const float4*>(kr + (i0 + e) * kGramPitch + d + 4);
+        k32[e] += dot4(kt, ki, dot4(kt4, ki4, 0.f));
+        q32[e] += dot4(qt, ki, dot4(qt4, ki4, 0.f));
       }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      kk[e] += k32[e];
+      qk[e] += q32[e];
     }
   }
   for (int h = hk * rep; h < (hk + 1) * rep; ++h) {
@@ -131,24 +198,27 @@ __global__ void __launch_bounds__(kGramWarps * 32) head_gram_kernel(const DeltaR
     __syncwarp();
     const float* g = decay[warp][0];
     const float beta_t = decay[warp][1][t];
-    float r = 1.f;                                   // g_(i+1) .. g_t, from i = t down to this lane's tokens
+    double r = 1.;                                   // g_(i+1) .. g_t, from i = t down to this lane's tokens
     for (int i = t - 1; i >= i0 + 8; --i) r *= g[i + 1];
+    float w[8];
 #pragma unroll
     for (int e = 7; e >= 0; --e) {
       const int i = i0 + e;
       if (i < t) r *= g[i + 1];
-      low[warp][t][i] = i < t ? beta_t * r * kk[e] : 0.f;
-      out[kW + t * kChunk + i] = i <= t ? r * qk[e] : 0.f;
+      low[warp][t][i] = i < t ? beta_t * (float)r * kk[e] : 0.f;
+      w[e] = (float)r * qk[e];
+      if (i == t) out[kDiag + kChunk + t] = qk[e];
     }
-    if (lane < kChunk) {
-      float p = 1.f, tail = 1.f;
+    put_coefs(out, 1, t, i0, w);
+    if (lane < kChunk) {                             // (rounded once: what a head forgets is common to all its state)
+      double p = 1., tail = 1.;
       for (int x = 0; x <= lane; ++x) p *= g[x];
       for (int x = lane + 1; x < kChunk; ++x) tail *= g[x];
-      out[kP + lane] = p;
-      out[kR + lane] = tail;
+      out[kP + lane] = (float)p;
+      out[kP + kChunk + lane] = (float)tail;
     }
     __syncwarp();
-    solve_columns(low[warp], decay[warp][1], out, lane);
+    solve(low[warp], decay[warp][1], out, lane);
   }
 }
 
@@ -163,7 +233,7 @@ __device__ __forceinline__ float4 load_four(const float* p, int d, int D, bool q
 template <int NG>
 __global__ void __launch_bounds__(kGramWarps * 32) channel_gram_kernel(const DeltaRule a) {
   US_PDL_PROLOGUE();
-  __shared__ float low[kGramWarps][kChunk][kChunk + 1], step[kGramWarps][kChunk];
+  __shared__ float low[kGramWarps][kChunk][kChunk + 1], read[kGramWarps][kChunk][kChunk + 1], step[kGramWarps][kChunk];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int s, start, n, chunk = blockIdx.x;
   const int h = blockIdx.y * kGramWarps + warp;
@@ -213,86 +283,262 @@ __global__ void __launch_bounds__(kGramWarps * 32) channel_gram_kernel(const Del
       }
     }
     if (lane < kChunk) low[warp][t][lane] = step[warp][t] * sum[0];
-    else out[kW + t * kChunk + lane - kChunk] = sum[0];
+    else read[warp][t][lane - kChunk] = sum[0];
+    if (lane == kChunk + t) out[kDiag + lane] = sum[0];
   }
   __syncwarp();
-  solve_columns(low[warp], step[warp], out, lane);
-}
-
-template <int BYTES>
-__device__ __forceinline__ void cp_async(float* dst, const float* src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-
-// x = hi + lo, hi rounded to TF32 (the product takes the upper 19 bits of lo).
-struct Split {
-  uint32_t hi, lo;
-  __device__ __forceinline__ Split() {}
-  __device__ __forceinline__ explicit Split(float x) {
-    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    lo = __float_as_uint(x - __uint_as_float(hi));
-  }
-};
-
-__device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_tf32_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-
-// An accumulator tile as the A operand of the next product: its columns 2 i and 2 i + 1 become k = i and i + 4.
-struct Tile {
-  Split s[4];
-  __device__ __forceinline__ Tile() {}
-  __device__ __forceinline__ explicit Tile(const float (&c)[4]) {
+  const int t = lane >> 1, i0 = (lane & 1) * 8;
+  float w[8];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) s[e] = Split(c[e]);
+  for (int e = 0; e < 8; ++e) w[e] = read[warp][t][i0 + e];
+  put_coefs(out, 1, t, i0, w);
+  solve(low[warp], step[warp], out, lane);
+}
+
+// An accumulator tile [16 x 8]: a lane's rows are r and r + 8, its columns 2 i and 2 i + 1.
+using Acc = f2[2];
+
+// An A operand [16 x 16] in three parts, from two accumulator tiles that stand side by side.
+struct Parts {
+  uint32_t p[3][4];
+  __device__ __forceinline__ Parts(const Acc& a, const Acc& b) {
+    uint32_t o[3];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const f2 x = (e < 2 ? a : b)[e & 1];
+      us::split3(lo2(x), hi2(x), o);
+#pragma unroll
+      for (int n = 0; n < 3; ++n) p[n][e] = o[n];
+    }
   }
 };
 
-// c = a b (first) or c += a b, all of them split: the products with low parts, the product of the high parts.  The
-// units add towards zero, so a sum takes all its low products before the first high one.
-__device__ __forceinline__ void mma_low(bool first, float (&c)[4], const Tile& a, const Split& b0, const Split& b1) {
-  if (first) mma_tf32_first(c, a.s[0].lo, a.s[2].lo, a.s[1].lo, a.s[3].lo, b0.hi, b1.hi);
-  else mma_tf32(c, a.s[0].lo, a.s[2].lo, a.s[1].lo, a.s[3].lo, b0.hi, b1.hi);
-  mma_tf32(c, a.s[0].hi, a.s[2].hi, a.s[1].hi, a.s[3].hi, b0.lo, b1.lo);
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_high(float (&c)[4], const Tile& a, const Split& b0, const Split& b1) {
-  mma_tf32(c, a.s[0].hi, a.s[2].hi, a.s[1].hi, a.s[3].hi, b0.hi, b1.hi);
+__device__ __forceinline__ void mma_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// Four B operands' tiles of one part, two to a load: tile n is b[n / 2][n % 2 * 2 ..]
+using Tiles = uint32_t[2][4];
+__device__ __forceinline__ void mma4(bool first, float (&c)[4][4], const uint32_t (&a)[4], const Tiles& b) {
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+    if (first) mma_first(c[n], a, b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
+    else mma(c[n], a, b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
+  }
+}
+// Products of `a` and four tiles, whose part p `load(b, p)` brings: high = those of the leading parts, low += the five
+// smaller ones (first: low = them).  Four sums side by side cover an instruction's latency.
+template <typename Load>
+__device__ __forceinline__ void products(bool first, float (&high)[4][4], float (&low)[4][4], const Parts& a, Load load) {
+  Tiles b;
+  load(b, 2);
+  mma4(first, low, a.p[0], b);
+  load(b, 1);
+  mma4(false, low, a.p[1], b);
+  mma4(false, low, a.p[0], b);
+  load(b, 0);
+  mma4(false, low, a.p[2], b);
+  mma4(false, low, a.p[1], b);
+  mma4(true, high, a.p[0], b);
 }
 
-// A chunk in shared memory: k of its tokens, q, with a decay per channel g (then the keys times R_t16), 32 columns of
-// v, the coefficients, P_16 per channel.  Rows of k, q, g and v stand 8 banks apart and rows of M and W 4 x 5: every
-// load below is then free of conflicts.
+// A chunk in shared memory, in bytes: arrays [part][token][channel] bf16 of k, of q and, with a decay per channel, of
+// k R_t16 (k and q then times P_t), rows 16 bytes past a multiple of 128; 32 columns of v (rows 4 banks apart); M and W
+// [part][t][i] (rows of 48 bytes); beta_t, W_tt, P_t and R_t16, or P_16 of every channel in place of the last two; the
+// last four tokens' k (k R_t16) whole, of sixteen channels those of a lane side by side.  Every load of them is free of conflicts.
+constexpr int kLast = 4;
 template <int DP, bool CHANNEL>
 struct Stage {
-  static constexpr int kD = DP + 8, kVp = kCols + 8, kMp = kChunk + 4;
-  static constexpr int kQ = kChunk * kD, kG = 2 * kChunk * kD, kV = (CHANNEL ? 3 : 2) * kChunk * kD;
-  static constexpr int kMat = kV + kChunk * kVp, kVec = kMat + 2 * kChunk * kMp, kAll = kVec + 2 * kChunk;
-  static constexpr int kFloats = kAll + (CHANNEL ? DP : 0);
+  static constexpr int kRow = (DP + 8) * 2, kPart = kChunk * kRow, kArray = 3 * kPart;
+  static constexpr int kQ = kArray, kKr = (CHANNEL ? 2 : 0) * kArray, kV = (CHANNEL ? 3 : 2) * kArray;
+  static constexpr int kVp = kCols + 4, kCoefs = kV + kChunk * kVp * 4, kCoefRow = 48, kCoefPart = kChunk * kCoefRow;
+  static constexpr int kVec = kCoefs + 6 * kCoefPart, kAll = kVec + 2 * kChunk * 4;
+  static constexpr int kTail = kAll + (CHANNEL ? DP : 2 * kChunk) * 4, kBytes = kTail + kLast * DP * 4;
 };
 
-// 4093 rows of 16 key and 32 value heads of 128 x 128, one sequence, with the coefficients: a decay per head 791 us four
-// tokens at a time, 457 here; a decay per channel 1513 us token by token, 582 here (two sequences of 4050: 1889,
-// 881).  64 sequences of five rows: 208 and 199 us before, 165 and 192 here.  The tensor pipe is busy for some 45 % of
-// it; the rest are the splits (three instructions a value) and the waits of a chunk's chain, one warp to a scheduler:
-// four warps to a tile's channels, each with the whole solve, took longer.
+// Named barriers.  Each has a second one for chunks of the other parity: a warp that arrives without waiting may be a
+// chunk ahead of those that wait, never two, since the next chunk but one is only laid out once this one is done with.
+enum Barrier : int { kTileBar = 1, kFullBar = 3, kEmptyBar = 5, kWritesBar = 7 };
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// What the warps of a chunk hand on: [chunk parity][tile][half of the channels][K S0, Q S0 of eight tokens][lane],
+// accumulator tiles over that half.  In place of the first two of the other half, once they are read, U.
+using Exchange = float4[2][kTiles][kSplit][4][32];
+
+// The warps that feed: a chunk's vectors are on their way to registers while the one before is multiplied.
 template <int DP, bool CHANNEL>
-__global__ void __launch_bounds__(kThreads, DP > 128 ? 1 : 2) chunk_delta_kernel(const DeltaRule a) {
+struct Feeder {
+  using St = Stage<DP, CHANNEL>;
+  static constexpr int kMine = kChunk * DP / 4 / kFeed;     // tokens of four channels
+  // With a decay per channel a thread has the same four channels of kMine tokens in turn, and the threads of a warp
+  // that share them stand kFours lanes apart; else it has pieces all over the chunk.
+  static constexpr int kFours = 32 * kMine / kChunk;
+  const DeltaRule& a;
+  const float *k, *q, *g, *v, *coef;
+  long long kstep, vstep, gstep;
+  int tid, T, col0, D;
+  bool quad;
+  float4 kv[kMine], qv[kMine], gv[CHANNEL ? kMine : 1], vv, cc[2];
+  __device__ __forceinline__ Feeder(const DeltaRule& a_, int tid_, int start, int s, int T_, int h, int hk, int col0_)
+      : a(a_), tid(tid_), T(T_), col0(col0_), D(a_.D) {
+    kstep = (long long)a.Hk * a.D;
+    vstep = (long long)a.H * a.V;
+    gstep = (long long)a.H * a.D;
+    k = a.k + ((long long)start * a.Hk + hk) * a.D;
+    q = a.q + ((long long)start * a.Hk + hk) * a.D;
+    g = a.g + ((long long)start * a.H + h) * a.D;
+    v = a.v + ((long long)start * a.H + h) * a.V;
+    coef = a.coef + (first_chunk(start, s) * a.H + h) * kCoef;
+    quad = (a.V & 3) == 0 && (a.D & 3) == 0;
+  }
+  __device__ __forceinline__ int token(int i) const {
+    return CHANNEL ? (tid & 31) / kFours * kMine + i : (tid + i * kFeed) / (DP / 4);
+  }
+  __device__ __forceinline__ int channel(int i) const {
+    return 4 * (CHANNEL ? (tid >> 5) * kFours + (tid & (kFours - 1)) : (tid + i * kFeed) % (DP / 4));
+  }
+  __device__ __forceinline__ void load(int chunk) {
+    const int t0 = chunk * kChunk, n = T - t0;
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) {
+      const int t = token(i), d = channel(i);
+      kv[i] = qv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (CHANNEL) gv[i] = make_float4(1.f, 1.f, 1.f, 1.f);
+      if (t < n && d < D) {
+        kv[i] = load_four(k + (t0 + t) * kstep, d, D, quad, 0.f);
+        qv[i] = load_four(q + (t0 + t) * kstep, d, D, quad, 0.f);
+        if (CHANNEL) gv[i] = load_four(g + (t0 + t) * gstep, d, D, quad, 1.f);
+      }
+    }
+    const int t = tid >> 3, c = col0 + (tid & 7) * 4;
+    vv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < n && c < a.V) vv = load_four(v + (t0 + t) * vstep, c, a.V, quad, 0.f);
+    const float4* m = reinterpret_cast<const float4*>(coef + (long long)chunk * a.H * kCoef);
+    cc[0] = m[tid];
+    if (tid < (CHANNEL ? kP : kCoef) / 4 - kFeed) cc[1] = m[tid + kFeed];
+  }
+  __device__ __forceinline__ static void put(unsigned char* at, const float4& x) {
+    uint32_t o[3], u[3];
+    split(x.x, x.y, o);
+    split(x.z, x.w, u);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(at + p * St::kPart) = make_uint2(o[p], u[p]);
+  }
+  __device__ __forceinline__ void last(unsigned char* b, int i, const float4& x) const {
+    const int t = token(i) - (kChunk - kLast), d = channel(i), at = t * DP + d / 16 * 16 + (d & 7) * 2 + (d & 8) / 4;
+    *reinterpret_cast<float2*>(b + St::kTail + at * 4) = make_float2(x.x, x.y);
+    *reinterpret_cast<float2*>(b + St::kTail + (at + 4) * 4) = make_float2(x.z, x.w);
+  }
+  __device__ __forceinline__ static float4 mul(const float4& x, const float4& y) {
+    return make_float4(x.x * y.x, x.y * y.y, x.z * y.z, x.w * y.w);
+  }
+  __device__ __forceinline__ void store(unsigned char* b) const {
+    const int d0 = channel(0);
+    float4 p, r;                                      // decays from the chunk's start, and to its end
+    if (CHANNEL) {
+      float4 all = make_float4(1.f, 1.f, 1.f, 1.f);   // of this thread's tokens
+      p = r = all;
+#pragma unroll
+      for (int i = 0; i < kMine; ++i) all = mul(all, gv[i]);
+      const int mine = (tid & 31) / kFours;
+#pragma unroll
+      for (int s = 0; s < 32 / kFours; ++s) {
+        const int from = s * kFours + (tid & (kFours - 1));
+        const float4 x = make_float4(__shfl_sync(0xffffffffu, all.x, from), __shfl_sync(0xffffffffu, all.y, from),
+                                     __shfl_sync(0xffffffffu, all.z, from), __shfl_sync(0xffffffffu, all.w, from));
+        if (s < mine) p = mul(p, x);
+        if (s > mine) r = mul(r, x);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) {
+      if (CHANNEL) p = mul(p, gv[i]);
+      unsigned char* at = b + token(i) * St::kRow + channel(i) * 2;
+      put(at, CHANNEL ? mul(kv[i], p) : kv[i]);
+      if (!CHANNEL && token(i) >= kChunk - kLast) last(b, i, kv[i]);
+      put(at + St::kQ, CHANNEL ? mul(qv[i], p) : qv[i]);
+    }
+    if (CHANNEL) {
+      if ((tid & 31) / kFours == 32 / kFours - 1) *reinterpret_cast<float4*>(b + St::kAll + d0 * 4) = p;
+#pragma unroll
+      for (int i = kMine - 1; i >= 0; --i) {
+        const float4 x = mul(kv[i], r);
+        put(b + St::kKr + token(i) * St::kRow + d0 * 2, x);
+        if (token(i) >= kChunk - kLast) last(b, i, x);
+        r = mul(r, gv[i]);
+      }
+    }
+    *reinterpret_cast<float4*>(b + St::kV + ((tid >> 3) * St::kVp + (tid & 7) * 4) * 4) = vv;
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const int e = tid + n * kFeed;                  // pieces of 16 bytes: two to a row of M and W
+      if (e < kDiag / 4) *reinterpret_cast<float4*>(b + St::kCoefs + (e >> 1) * St::kCoefRow + (e & 1) * 16) = cc[n];
+      else if (e < (CHANNEL ? kP : kCoef) / 4) *reinterpret_cast<float4*>(b + St::kVec + (e - kDiag / 4) * 16) = cc[n];
+    }
+  }
+  // O = P Q S0 + W U of eight of a chunk's tokens and sixteen columns
+  __device__ __forceinline__ void read_out(const unsigned char* b, const Exchange& ex, int chunk, float* out) const {
+    const int warp = tid >> 5, lane = tid & 31, tile = warp / kSplit, half = warp % kSplit, r = lane >> 2, i = lane & 3;
+    const float4(*parts)[4][32] = ex[chunk & 1][tile];
+    const float4(*u)[32] = parts[half ^ 1];
+    const float4 seen0 = parts[0][2 + half][lane], seen1 = parts[1][2 + half][lane], u0 = u[0][lane], u1 = u[1][lane];
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(b) + St::kCoefs + 3 * St::kCoefPart +
+                        (half * 8 + (lane & 7)) * St::kCoefRow + ((lane >> 3) & 1) * 16;
+    uint32_t w01[4], w22[4];
+    us::ldsm4(w01, at + (lane >> 4) * St::kCoefPart);                 // two parts
+    us::ldsm4(w22, at + 2 * St::kCoefPart);
+    const float* vec = reinterpret_cast<const float*>(b + St::kVec) + kChunk + half * 8 + 2 * i;
+    const float2 diag = *reinterpret_cast<const float2*>(vec);
+    const float2 p = CHANNEL ? make_float2(1.f, 1.f) : *reinterpret_cast<const float2*>(vec + kChunk);
+    const Acc ua = {pack2(u0.x, u0.y), pack2(u0.z, u0.w)}, ub = {pack2(u1.x, u1.y), pack2(u1.z, u1.w)};
+    float o[4];
+    const Parts up(ua, ub);
+    float a1[4], a2[4];
+    mma_first(a2, up.p[0], w22[0], w22[1]);
+    mma_first(a1, up.p[0], w01[2], w01[3]);
+    mma_first(o, up.p[0], w01[0], w01[1]);
+    mma(a2, up.p[1], w01[2], w01[3]);
+    mma(a1, up.p[1], w01[0], w01[1]);
+    mma(a2, up.p[2], w01[0], w01[1]);
+    const float4 mine = half ? u1 : u0;
+    o[0] = fmaf(diag.x, mine.x, o[0] + (a1[0] + a2[0]));
+    o[1] = fmaf(diag.y, mine.y, o[1] + (a1[1] + a2[1]));
+    o[2] = fmaf(diag.x, mine.z, o[2] + (a1[2] + a2[2]));
+    o[3] = fmaf(diag.y, mine.w, o[3] + (a1[3] + a2[3]));
+    const float seen[4] = {seen0.x + seen1.x, seen0.y + seen1.y, seen0.z + seen1.z, seen0.w + seen1.w};
+    const int col = col0 + tile * 16 + r;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int t = chunk * kChunk + half * 8 + 2 * i + (c & 1), v = col + (c >> 1) * 8;
+      if (t < T && v < a.V) out[t * vstep + v] = fmaf(seen[c], (c & 1) ? p.y : p.x, o[c]);
+    }
+  }
+};
+
+// 4093 rows of 16 key and 32 value heads of 128 x 128, one sequence, with the coefficients: a decay per head 790 us four
+// tokens at a time, 522 here; a decay per channel 1516 us token by token, 618 here (two sequences of 4050: 1146 -> 930,
+// 1887 -> 1122).  Operands in two TF32 parts and three products took 456 and 582, but left results up to 3.1 times as
+// far from 64 bits as the FP32 recurrence's; this form's are 0.5 to 1.05 of it (state 1.15 where a token forgets half).
+// What bounds it is the chain: 162 tensor instructions of a warp take 1300 of a chunk's 3700 clocks; the rest are the
+// splits (eleven instructions a pair of values) and waits, one warp of the chain to a scheduler.
+template <int DP, bool CHANNEL, int PER_SM>
+__global__ void __launch_bounds__(kThreads, PER_SM) chunk_delta_kernel(const DeltaRule a) {
   US_PDL_PROLOGUE();
   using St = Stage<DP, CHANNEL>;
   constexpr int kOwn = DP / kSplit, NJ = kOwn / 16;   // channels of a warp, in pairs of eight-wide tiles
-  extern __shared__ __align__(16) float sm[];
-  __shared__ __align__(16) float4 parts[2][kTiles][kSplit][4][32];
+  extern __shared__ __align__(128) unsigned char sm[];
+  __shared__ __align__(16) Exchange exchange;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y, s = blockIdx.z, hk = h / (a.H / a.Hk), col0 = blockIdx.x * kCols;
   const int start = a.cu[s], T = a.cu[s + 1] - start, slot = a.slots[s];
@@ -305,272 +551,222 @@ __global__ void __launch_bounds__(kThreads, DP > 128 ? 1 : 2) chunk_delta_kernel
     return;
   }
   const int chunks = (T + kChunk - 1) / kChunk;
-  if (a.D < DP || col0 + kCols > a.V || (T % kChunk) != 0) {      // places that no copy fills: zero
-    for (int e = tid; e < kBufs * St::kFloats; e += kThreads) sm[e] = 0.f;
-    __syncthreads();
-  }
-  const bool quad = (a.V & 3) == 0 && (a.D & 3) == 0;
-  const long long kstep = (long long)a.Hk * a.D, vstep = (long long)a.H * a.V, gstep = (long long)a.H * a.D;
-  const float* kg = a.k + ((long long)start * a.Hk + hk) * a.D;
-  const float* qg = a.q + ((long long)start * a.Hk + hk) * a.D;
-  const float* gg = a.g + ((long long)start * a.H + h) * a.D;               // per channel
-  const float* vg = a.v + ((long long)start * a.H + h) * a.V + col0;
-  const float* cg = a.coef + (first_chunk(start, s) * a.H + h) * kCoef;
-  auto fetch = [&](int chunk) {                       // (an empty group past the end)
-    if (chunk < chunks) {
-      float* dst = sm + (chunk % kBufs) * St::kFloats;
-      const int t0 = chunk * kChunk, n = min(kChunk, T - t0);
-      if (quad) {
-        for (int t = warp; t < n; t += kThreads / 32)
-#pragma unroll
-          for (int d = lane * 4; d < DP; d += 128)
-            if (d < a.D) {
-              cp_async<16>(dst + t * St::kD + d, kg + (t0 + t) * kstep + d);
-              cp_async<16>(dst + St::kQ + t * St::kD + d, qg + (t0 + t) * kstep + d);
-              if (CHANNEL) cp_async<16>(dst + St::kG + t * St::kD + d, gg + (t0 + t) * gstep + d);
-            }
-        const int c = (lane & 7) * 4;
-        for (int t = tid >> 3; t < n; t += kThreads / 8)
-          if (col0 + c < a.V) cp_async<16>(dst + St::kV + t * St::kVp + c, vg + (t0 + t) * vstep + c);
-      } else {
-        for (int t = warp; t < n; t += kThreads / 32) {
-          for (int d = lane; d < a.D; d += 32) {
-            cp_async<4>(dst + t * St::kD + d, kg + (t0 + t) * kstep + d);
-            cp_async<4>(dst + St::kQ + t * St::kD + d, qg + (t0 + t) * kstep + d);
-            if (CHANNEL) cp_async<4>(dst + St::kG + t * St::kD + d, gg + (t0 + t) * gstep + d);
-          }
-          if (col0 + lane < a.V) cp_async<4>(dst + St::kV + t * St::kVp + lane, vg + (t0 + t) * vstep + lane);
-        }
-      }
-      const float* src = cg + (long long)chunk * a.H * kCoef;
-#pragma unroll
-      for (int e = tid * 4; e < 2 * kChunk * kChunk; e += kThreads * 4)      // both matrices, row by row
-        cp_async<16>(dst + St::kMat + e / kChunk * St::kMp + e % kChunk, src + e);
-      if (!CHANNEL && tid < 2 * kChunk / 4) cp_async<16>(dst + St::kVec + tid * 4, src + kP + tid * 4);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // keys and queries times P_t, keys times R_t16 in the decays' place, P_16; a thread per channel
-  auto decayed = [&](int chunk) {
-    float* b = sm + (chunk % kBufs) * St::kFloats;
-    const int n = min(kChunk, T - chunk * kChunk);
-    for (int d = tid; d < DP; d += kThreads) {
-      float g[kChunk], k[kChunk], p = 1.f, r = 1.f;
-#pragma unroll
-      for (int t = 0; t < kChunk; ++t) {
-        const bool in = t < n && d < a.D;
-        g[t] = in ? b[St::kG + t * St::kD + d] : 1.f;
-        k[t] = in ? b[t * St::kD + d] : 0.f;
-        p *= g[t];
-        b[t * St::kD + d] = k[t] * p;
-        b[St::kQ + t * St::kD + d] *= p;
-      }
-      b[St::kAll + d] = p;
-#pragma unroll
-      for (int t = kChunk - 1; t >= 0; --t) {
-        b[St::kG + t * St::kD + d] = k[t] * r;
-        r *= g[t];
-      }
-    }
-  };
+  if (tid >= kCompute) {
+    Feeder<DP, CHANNEL> feed(a, tid - kCompute, start, s, T, h, hk, col0);
+    float* out = a.out + ((long long)start * a.H + h) * a.V;
+    feed.load(0);
 #pragma unroll 1
-  for (int f = 0; f < kBufs - 1; ++f) fetch(f);
+    for (int ch = 0; ch <= chunks; ++ch) {
+      if (ch < chunks) {
+        if (ch >= 2) bar_sync(kEmptyBar + (ch & 1), kThreads);
+        feed.store(sm + (ch & 1) * St::kBytes);
+        bar_arrive(kFullBar + (ch & 1), kThreads);
+        if (ch + 1 < chunks) feed.load(ch + 1);
+      }
+      if (ch == 0) continue;
+      bar_sync(kWritesBar + ((ch - 1) & 1) * (kCompute / 32) + warp - kCompute / 32, 64);
+      feed.read_out(sm + ((ch - 1) & 1) * St::kBytes, exchange, ch - 1, out);
+    }
+    return;
+  }
   const int tile = warp / kSplit, half = warp % kSplit, r = lane >> 2, i = lane & 3;
-  // A tile's columns 2 i and 2 i + 1 are tokens i and 4 + (i ^ 2) of eight: loads of rows by column number and by
-  // column pair then both meet every bank once.
-  const int t0 = i, t1 = 4 + (i ^ 2), tr = (r & 1) ? 4 + ((r >> 1) ^ 2) : r >> 1;
-  const int col = col0 + tile * 16 + r, dbase = half * kOwn;
+  const int cl = tile * 16 + r, col = col0 + cl, dbase = half * kOwn;
   float* Sg = a.state + ((long long)slot * a.H + h) * a.D * a.V;
   const bool fresh = a.pos && a.pos[start] == 0;
-  // S^T: tile (j, e) has columns n = channel 16 j + 2 n + e of the warp's
-  float S[NJ][2][4];
+  // S^T: tile (j, e) has channels 16 j + 8 e .. of the warp's; a lane's are 2 i and 2 i + 1 of them
+  Acc S[NJ][2];
 #pragma unroll
   for (int j = 0; j < NJ; ++j)
 #pragma unroll
     for (int e = 0; e < 2; ++e)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int d = dbase + 16 * j + 4 * i + 2 * (c & 1) + e, v = col + (c >> 1) * 8;
-        S[j][e][c] = !fresh && d < a.D && v < a.V ? Sg[(long long)d * a.V + v] : 0.f;
+      for (int c = 0; c < 2; ++c) {
+        const int d = dbase + 16 * j + 8 * e + 2 * i, v = col + c * 8;
+        const bool in = !fresh && v < a.V;
+        const float* p = Sg + (long long)d * a.V + v;
+        S[j][e][c] = pack2(in && d < a.D ? p[0] : 0.f, in && d + 1 < a.D ? p[a.V] : 0.f);
       }
-  float* op = a.out + ((long long)start * a.H + h) * a.V + col;
-  const long long ostep = (long long)a.H * a.V;
-  if (CHANNEL) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 2) : "memory");
-    __syncthreads();
-    decayed(0);
-  }
+  const uint32_t base0 = (uint32_t)__cvta_generic_to_shared(sm);
+  // places of a lane's rows: [n = token][k = channel] operands, [k = token][n = channel] ones, M
+  const uint32_t at_x = ((lane & 7) + (lane >> 4) * 8) * St::kRow + (dbase + ((lane >> 3) & 1) * 8) * 2;
+  const uint32_t at_s = St::kKr + (lane & 15) * St::kRow + (dbase + (lane >> 4) * 8) * 2;
+  const uint32_t at_m = St::kCoefs + ((lane & 7) + (lane >> 4) * 8) * St::kCoefRow + ((lane >> 3) & 1) * 16;
+#pragma unroll 1
   for (int ch = 0; ch < chunks; ++ch) {
-    // this chunk's vectors are there (decayed ones: and the next chunk's), the one before is consumed
-    asm volatile("cp.async.wait_group %0;" ::"n"(CHANNEL ? 0 : kBufs - 2) : "memory");
-    __syncthreads();
-    fetch(ch + kBufs - 1);
-    if (CHANNEL && ch + 1 < chunks) decayed(ch + 1);
-    const float* base = sm + (ch % kBufs) * St::kFloats;
-    const float* M = base + St::kMat;
-    const float* vec = base + St::kVec;
-    // What keys (tiles 0, 1) and queries (2, 3) see of S0, over this warp's channels.  As the units add towards
-    // zero, no sum of theirs is longer than two steps of channels; longer ones and the state's are rounded.
-    float x[4][4];
+    bar_sync(kFullBar + (ch & 1), kThreads);
+    const unsigned char* base = sm + (ch & 1) * St::kBytes;
+    const uint32_t addr = base0 + (ch & 1) * St::kBytes;
+    // what keys (tiles 0, 1) and queries (2, 3) see of S0, over this warp's channels
+    Acc x[4];
+    float low[4][4];
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
-      const Tile s0(S[j][0]), s1(S[j][1]);
-      float4 f[4];
-#pragma unroll
-      for (int n = 0; n < 4; ++n)
-        f[n] = *reinterpret_cast<const float4*>(base + (n >> 1) * St::kQ + ((n & 1) * 8 + tr) * St::kD + dbase + 16 * j + 4 * i);
+      const Parts sp(S[j][0], S[j][1]);
       float y[4][4];
+      products(j == 0, y, low, sp, [&](Tiles& b, int p) {
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const Split bx(f[n].x), by(f[n].y), bz(f[n].z), bw(f[n].w);
-        mma_low(true, y[n], s0, bx, bz);
-        mma_low(false, y[n], s1, by, bw);
-        mma_high(y[n], s0, bx, bz);
-        mma_high(y[n], s1, by, bw);
-      }
+        for (int w = 0; w < 2; ++w) us::ldsm4(b[w], addr + at_x + w * St::kQ + p * St::kPart + j * 32);
+      });
 #pragma unroll
       for (int n = 0; n < 4; ++n)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) x[n][c] = j ? x[n][c] + y[n][c] : y[n][c];
+        for (int c = 0; c < 2; ++c) {
+          const f2 z = pack2(y[n][2 * c], y[n][2 * c + 1]);
+          x[n][c] = j ? add2(x[n][c], z) : z;
+        }
     }
-    float4(*mine)[32] = parts[ch & 1][tile][half];
+    float4(*mine)[32] = exchange[ch & 1][tile][half];
+    float4(*other)[32] = exchange[ch & 1][tile][half ^ 1];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) mine[n][lane] = make_float4(x[n][0], x[n][1], x[n][2], x[n][3]);
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + tile), "n"(32 * kSplit) : "memory");
+    for (int n = 0; n < 4; ++n) {
 #pragma unroll
-    for (int o = 1; o < kSplit; ++o) {
-      const float4(*other)[32] = parts[ch & 1][tile][(half + o) % kSplit];
+      for (int c = 0; c < 2; ++c) x[n][c] = add2(x[n][c], pack2(low[n][2 * c], low[n][2 * c + 1]));
+      mine[n][lane] = make_float4(lo2(x[n][0]), hi2(x[n][0]), lo2(x[n][1]), hi2(x[n][1]));
+    }
+    const float* v = reinterpret_cast<const float*>(base + St::kV);
+    const float* vec = reinterpret_cast<const float*>(base + St::kVec);
+    const float* decay = reinterpret_cast<const float*>(base + St::kAll);
+    f2 beta[2], rest[2];                              // beta_t, R_t16 of tokens 2 i, 2 i + 1 of eight
+    Acc w[2], u[2];
+    uint32_t m[3][4];
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        if (n >= 2 && n % kSplit != half) continue;   // queries of another warp's tokens
-        const float4 y = other[n][lane];
-        x[n][0] += y.x;
-        x[n][1] += y.y;
-        x[n][2] += y.z;
-        x[n][3] += y.w;
+    for (int n = 0; n < 2; ++n) {
+      beta[n] = *reinterpret_cast<const f2*>(vec + n * 8 + 2 * i);
+      rest[n] = CHANNEL ? 0 : *reinterpret_cast<const f2*>(decay + kChunk + n * 8 + 2 * i);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float* at = v + (n * 8 + 2 * i) * St::kVp + cl + c * 8;
+        w[n][c] = pack2(at[0], at[St::kVp]);
       }
     }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) us::ldsm4(m[q], addr + at_m + q * St::kCoefPart);
+    bar_sync(kTileBar + tile, 32 * kSplit);
     // U = M (V - P X)
-    Tile res[2];
-    float p[2][2];
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
-      p[n][0] = CHANNEL ? 1.f : vec[n * 8 + t0];
-      p[n][1] = CHANNEL ? 1.f : vec[n * 8 + t1];
-      float w[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        w[c] = fmaf(-p[n][c & 1], x[n][c],
-                    base[St::kV + (n * 8 + ((c & 1) ? t1 : t0)) * St::kVp + tile * 16 + r + (c >> 1) * 8]);
-      res[n] = Tile(w);
+      const float4 y = other[n][lane];
+      const f2 minus = CHANNEL ? pack2(-1.f, -1.f) : mul2(*reinterpret_cast<const f2*>(decay + n * 8 + 2 * i), pack2(-1.f, -1.f));
+      w[n][0] = fma2(minus, add2(x[n][0], pack2(y.x, y.y)), w[n][0]);
+      w[n][1] = fma2(minus, add2(x[n][1], pack2(y.z, y.w)), w[n][1]);
     }
-    float u[2][4], u1[4];
-    const float* at = M + tr * St::kMp;
-    const Split m0(at[t0]), m1(at[t1]), m2(at[8 * St::kMp + t0]), m3(at[8 * St::kMp + t1]);
-    const Split m4(at[8 * St::kMp + 8 + t0]), m5(at[8 * St::kMp + 8 + t1]);
-    mma_low(true, u[0], res[0], m0, m1);
-    mma_low(true, u[1], res[0], m2, m3);
-    mma_low(true, u1, res[1], m4, m5);
-    mma_high(u[0], res[0], m0, m1);
-    mma_high(u[1], res[0], m2, m3);
-    mma_high(u1, res[1], m4, m5);
+    {
+      const Parts wp(w[0], w[1]);
+      float a0[2][4], a1[2][4], a2[2][4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) u[1][c] += u1[c];
-    const Tile ut[2] = {Tile(u[0]), Tile(u[1])};
-    // S' = P_16 S0 + (R K)^T U
-    Tile wr[2];
+      for (int n = 0; n < 2; ++n) mma_first(a2[n], wp.p[0], m[2][n * 2], m[2][n * 2 + 1]);
 #pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      if (CHANNEL) {
-        wr[n] = ut[n];
-      } else {
-        const float r0 = vec[kChunk + n * 8 + t0], r1 = vec[kChunk + n * 8 + t1];
-        const float w[4] = {u[n][0] * r0, u[n][1] * r1, u[n][2] * r0, u[n][3] * r1};
-        wr[n] = Tile(w);
-      }
-    }
-    const float* kr = base + (CHANNEL ? St::kG : 0);
+      for (int n = 0; n < 2; ++n) mma_first(a1[n], wp.p[0], m[1][n * 2], m[1][n * 2 + 1]);
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      float y[2][4];
-      Split b[2][2][2];
+      for (int n = 0; n < 2; ++n) mma_first(a0[n], wp.p[0], m[0][n * 2], m[0][n * 2 + 1]);
 #pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        const float2 f0 = *reinterpret_cast<const float2*>(kr + (n * 8 + t0) * St::kD + dbase + 16 * j + 2 * r);
-        const float2 f1 = *reinterpret_cast<const float2*>(kr + (n * 8 + t1) * St::kD + dbase + 16 * j + 2 * r);
-        b[n][0][0] = Split(f0.x);
-        b[n][0][1] = Split(f1.x);
-        b[n][1][0] = Split(f0.y);
-        b[n][1][1] = Split(f1.y);
+      for (int n = 0; n < 2; ++n) mma(a2[n], wp.p[1], m[1][n * 2], m[1][n * 2 + 1]);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) mma_low(n == 0, y[e], wr[n], b[n][e][0], b[n][e][1]);
-      }
+      for (int n = 0; n < 2; ++n) mma(a1[n], wp.p[1], m[0][n * 2], m[0][n * 2 + 1]);
+#pragma unroll
+      for (int n = 0; n < 2; ++n) mma(a2[n], wp.p[2], m[0][n * 2], m[0][n * 2 + 1]);
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) mma_high(y[e], wr[n], b[n][e][0], b[n][e][1]);
-      float4 all;
-      if (CHANNEL) all = *reinterpret_cast<const float4*>(base + St::kAll + dbase + 16 * j + 4 * i);
-      else all.x = all.y = all.z = all.w = vec[kChunk - 1];
+        for (int c = 0; c < 2; ++c) {
+          const f2 sum = add2(pack2(a1[n][2 * c], a1[n][2 * c + 1]), pack2(a2[n][2 * c], a2[n][2 * c + 1]));
+          u[n][c] = fma2(beta[n], w[n][c], add2(pack2(a0[n][2 * c], a0[n][2 * c + 1]), sum));
+        }
+    }
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        S[j][0][c] = fmaf(S[j][0][c], (c & 1) ? all.z : all.x, y[0][c]);
-        S[j][1][c] = fmaf(S[j][1][c], (c & 1) ? all.w : all.y, y[1][c]);
+    for (int n = 0; n < 2; ++n) other[n][lane] = make_float4(lo2(u[n][0]), hi2(u[n][0]), lo2(u[n][1]), hi2(u[n][1]));
+    bar_arrive(kWritesBar + (ch & 1) * (kCompute / 32) + warp, 64);
+    // S' = P_16 S0 + (R K)^T U
+    {
+      // The last four tokens, which carry most of a state that decays fast, on the FP32 units: beside them the tensor
+      // cores' sums would cut more of the others off.
+      f2 last[kLast][2];
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          if (!CHANNEL) u[n][c] = mul2(u[n][c], rest[n]);
+          if (n == 1) {
+#pragma unroll
+            for (int t = 0; t < kLast; ++t) {
+              const float z = __shfl_sync(0xffffffffu, (t & 1) ? hi2(u[1][c]) : lo2(u[1][c]), (lane & ~3) | (2 + (t >> 1)));
+              last[t][c] = pack2(z, z);
+            }
+            if (i >= 2) u[1][c] = 0;
+          }
+        }
+      const Parts up(u[0], u[1]);
+      const float* tail = reinterpret_cast<const float*>(base + St::kTail) + dbase + 4 * i;
+      const float all = CHANNEL ? 0.f : decay[kChunk - 1];
+#pragma unroll
+      for (int j = 0; j < NJ; j += 2) {               // two sixteens of channels
+        float y[4][4];
+        products(true, y, low, up, [&](Tiles& b, int q) {
+#pragma unroll
+          for (int f = 0; f < 2; ++f) us::ldsm4t(b[f], addr + at_s + q * St::kPart + (j + f) * 32);
+        });
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+          f2 k[kLast][2];                             // a lane's channels of both tiles
+#pragma unroll
+          for (int t = 0; t < kLast; ++t) lds_vec(k[t], tail + t * DP + 16 * (j + f));
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int n = 2 * f + e;
+            Acc& x0 = S[j + f][e];
+            const f2 g = CHANNEL ? *reinterpret_cast<const f2*>(decay + dbase + 16 * (j + f) + 8 * e + 2 * i) : pack2(all, all);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              x0[c] = add2(fma2(x0[c], g, pack2(low[n][2 * c], low[n][2 * c + 1])), pack2(y[n][2 * c], y[n][2 * c + 1]));
+#pragma unroll
+              for (int t = 0; t < kLast; ++t) x0[c] = fma2(k[t][e], last[t][c], x0[c]);
+            }
+          }
+        }
       }
     }
-    // O = P Q S0 + W U: a tile of eight tokens per warp
-    const float* W = M + kChunk * St::kMp;
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      if (n % kSplit != half) continue;
-      float o[4];
-      Split b[2][2];
-#pragma unroll
-      for (int m = 0; m <= n; ++m) {
-        const float* wt = W + (n * 8 + tr) * St::kMp + m * 8;
-        b[m][0] = Split(wt[t0]);
-        b[m][1] = Split(wt[t1]);
-        mma_low(m == 0, o, ut[m], b[m][0], b[m][1]);
-      }
-#pragma unroll
-      for (int m = 0; m <= n; ++m) mma_high(o, ut[m], b[m][0], b[m][1]);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int t = ch * kChunk + n * 8 + ((c & 1) ? t1 : t0);
-        if (t < T && col + (c >> 1) * 8 < a.V) op[t * ostep + (c >> 1) * 8] = fmaf(x[2 + n][c], p[n][c & 1], o[c]);
-      }
-    }
+    if (ch + 2 < chunks) bar_arrive(kEmptyBar + (ch & 1), kThreads);
   }
 #pragma unroll
   for (int j = 0; j < NJ; ++j)
 #pragma unroll
     for (int e = 0; e < 2; ++e)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int d = dbase + 16 * j + 4 * i + 2 * (c & 1) + e, v = col + (c >> 1) * 8;
-        if (d < a.D && v < a.V) Sg[(long long)d * a.V + v] = S[j][e][c];
+      for (int c = 0; c < 2; ++c) {
+        const int d = dbase + 16 * j + 8 * e + 2 * i, v = col + c * 8;
+        float* p = Sg + (long long)d * a.V + v;
+        if (v < a.V && d < a.D) p[0] = lo2(S[j][e][c]);
+        if (v < a.V && d + 1 < a.D) p[a.V] = hi2(S[j][e][c]);
       }
+}
+
+template <int DP, bool CHANNEL, int PER_SM>
+int launch(const DeltaRule& a, dim3 grid, int smem, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    US_CUDA_CHECK(cudaFuncSetAttribute(chunk_delta_kernel<DP, CHANNEL, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    configured = true;
+  }
+  US_CUDA_CHECK(us::launch_pdl(chunk_delta_kernel<DP, CHANNEL, PER_SM>, grid, dim3(kThreads), smem, stream, a));
+  return US_OK;
 }
 
 template <int DP, bool CHANNEL>
 int launch(const DeltaRule& a, cudaStream_t stream) {
-  constexpr int need = kBufs * Stage<DP, CHANNEL>::kFloats * sizeof(float);
+  constexpr int need = 2 * Stage<DP, CHANNEL>::kBytes;
   constexpr int alone = need > 110 * 1024 ? need : 110 * 1024;      // shared memory that one CTA per SM has
-  static bool configured = false;
   static int sms = 0;
-  if (!configured) {
+  if (!sms) {
     int dev = 0;
     US_CUDA_CHECK(cudaGetDevice(&dev));
     US_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    US_CUDA_CHECK(cudaFuncSetAttribute(chunk_delta_kernel<DP, CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, alone));
-    configured = true;
   }
   // CTAs that are launched while the kernel before still runs would be packed two to an SM where it
-  // leaves room: with fewer CTAs than SMs each asks for more shared memory than half an SM has
+  // leaves room: with fewer CTAs than SMs each asks for more shared memory than half an SM has, and may have more
+  // registers (4093 rows, 32 heads of 128 x 128: 128 registers 587 us, 204 531)
   const dim3 grid(us::ceil_div(a.V, kCols), a.H, a.B);
-  const size_t smem = (long long)grid.x * grid.y * grid.z <= sms ? alone : need;
-  US_CUDA_CHECK(us::launch_pdl(chunk_delta_kernel<DP, CHANNEL>, grid, dim3(kThreads), smem, stream, a));
-  return US_OK;
+  if ((long long)grid.x * grid.y * grid.z <= sms) return launch<DP, CHANNEL, 1>(a, grid, alone, stream);
+  return launch<DP, CHANNEL, (DP > 128 ? 1 : 2)>(a, grid, need, stream);
 }
 
 int run(const DeltaRule& a, int rows, bool channel, cudaStream_t stream) {

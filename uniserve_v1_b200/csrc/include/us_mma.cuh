@@ -37,6 +37,16 @@ __device__ __forceinline__ uint32_t pack_bf(float a, float b) {
   __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&p);
 }
+// (x, y) = sum of three bf16 pairs
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&o)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+    o[i] = *reinterpret_cast<const uint32_t*>(&p);
+    x -= bf2f(p.x);
+    y -= bf2f(p.y);
+  }
+}
 // byte offset of 16-byte piece c of row r in a tile whose rows hold `pieces` (a multiple of 8):
 // pieces are XOR-swizzled by row so that 8 consecutive rows read 8 different bank groups
 __device__ __forceinline__ uint32_t swz(int r, int c, int pieces) {

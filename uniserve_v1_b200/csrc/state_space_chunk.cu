@@ -52,17 +52,6 @@ __device__ __forceinline__ float softplus_f(float x) {
 // byte offset of piece c (of four) of row r: 8 rows of one piece hit 8 bank groups
 __device__ __forceinline__ uint32_t swz4(int r, int c) { return (uint32_t)(r * 4 + (c ^ ((r >> 1) & 3))) * 16u; }
 
-// (x, y) = sum of three bf16 pairs
-__device__ __forceinline__ void split3(float x, float y, uint32_t (&o)[3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
-    o[i] = *reinterpret_cast<const uint32_t*>(&p);
-    x -= us::bf2f(p.x);
-    y -= us::bf2f(p.y);
-  }
-}
-
 // One warp: exponents of the chunk whose raw step sizes its lanes hold (tokens 2 lane, 2 lane + 1).
 // With `fixed`, *fixed is every token's exponent.
 __device__ __forceinline__ void form_exponents(Exponents& x, float raw0, float raw1, int n, float A,
@@ -191,7 +180,7 @@ __global__ void __launch_bounds__(kThreads, 1) state_space_chunk_kernel(const Ch
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         uint32_t q[3];
-        split3(us::bf2f(v.b[2 * e]) * w, us::bf2f(v.b[2 * e + 1]) * w, q);
+        us::split3(us::bf2f(v.b[2 * e]) * w, us::bf2f(v.b[2 * e + 1]) * w, q);
 #pragma unroll
         for (int i = 0; i < 3; ++i) o[i][e] = q[i];
       }
@@ -204,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1) state_space_chunk_kernel(const Ch
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           uint32_t q[3];
-          split3(S[t][2 * e], S[t][2 * e + 1], q);
+          us::split3(S[t][2 * e], S[t][2 * e + 1], q);
           const uint32_t d = ss + swz4(sm_ + r0 + e * 8, sn + t) + cq * 2;
 #pragma unroll
           for (int i = 0; i < 3; ++i)
@@ -275,9 +264,9 @@ __global__ void __launch_bounds__(kThreads, 1) state_space_chunk_kernel(const Ch
           const float h0 = x.hi[s0], l0 = x.lo[s0], h1 = x.hi[s0 + 1], l1 = x.lo[s0 + 1];
           const float d0 = x.dt[s0], d1 = x.dt[s0 + 1];
           const float (&q)[4] = sc[2 * k + e];
-          split3(s0 <= ta ? q[0] * (expf((ha - h0) + (la - l0)) * d0) : 0.f,
+          us::split3(s0 <= ta ? q[0] * (expf((ha - h0) + (la - l0)) * d0) : 0.f,
                  s0 + 1 <= ta ? q[1] * (expf((ha - h1) + (la - l1)) * d1) : 0.f, m[2 * e]);
-          split3(s0 <= tb ? q[2] * (expf((hb - h0) + (lb - l0)) * d0) : 0.f,
+          us::split3(s0 <= tb ? q[2] * (expf((hb - h0) + (lb - l0)) * d0) : 0.f,
                  s0 + 1 <= tb ? q[3] * (expf((hb - h1) + (lb - l1)) * d1) : 0.f, m[2 * e + 1]);
         }
 #pragma unroll
