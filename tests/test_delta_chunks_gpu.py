@@ -89,3 +89,37 @@ def test_no_further_off_than_fp32(T, D, V, rate, per_channel):
     off = lambda a, b: float((a.double() - b).norm() / b.norm())
     assert off(got, want) < 1.17 * off(plain, want)
     assert off(S[0], state[0]) < 1.17 * off(plain_state, state[0])
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+@pytest.mark.parametrize("where", ["v", "k", "q", "g"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_not_finite_stays_with_later_tokens(where, bad, per_channel):
+    """A token that is not finite in the middle of a chunk: tokens before it, and for a value the other columns, are what
+    they are without it."""
+    from uniserve_v1_b200.ops import vector_delta as VD
+    T, at, head, D, V = 40, 21, 1, 64, 40
+    i32 = dict(dtype=torch.int32, device="cuda")
+    m = VD.SeqMeta(torch.tensor([0, T], **i32), torch.zeros(1, **i32), torch.arange(T, **i32) + 7, False)
+    outs = []
+    for spoiled in (False, True):
+        q, k, v, g, beta, S = _inputs([T], 2, 2, D, V, 0.3, per_channel)
+        if spoiled:
+            x = dict(q=q, k=k, v=v, g=g)[where]
+            x[(at, head) if x.dim() == 2 else (at, head, 5)] = bad
+        S = S[:1].contiguous()
+        outs.append((VD.vector_delta_rule(q, k, v, g, S, m, beta=beta), S))
+    (clean, S0), (got, S1) = outs
+    # the sums of a tile without its later tokens are taken in another order: FP32 sums of 16 products
+    near = lambda a, b: torch.allclose(a, b, rtol=0, atol=16 * 2.0 ** -24 * float(clean.abs().max()))
+    assert near(got[:at], clean[:at]) and torch.equal(got[:, 0], clean[:, 0])
+    if where == "v":
+        others = [c for c in range(V) if c != 5]
+        assert near(got[:, head, others], clean[:, head, others])
+        assert not bool(torch.isfinite(got[at:, head, 5]).any()) and not bool(torch.isfinite(S1[0, head, :, 5]).any())
+        assert bool(torch.isfinite(S1[0, head][:, others]).all())
+    elif where == "q":
+        assert near(got[at + 1:], clean[at + 1:]) and torch.equal(S1, S0)
+        assert not bool(torch.isfinite(got[at, head]).any())
+    else:
+        assert not bool(torch.isfinite(got[at:, head]).any())

@@ -30,6 +30,10 @@
 // in shared memory, two chunks at most, and they form a chunk's outputs while the next one is under way.  A sequence
 // whose first packed row stands at position 0 starts from a zero state whatever its slot holds; a negative slot marks
 // padding.
+//
+// Values that are not finite stay where the recurrence has them.  M and W are lower triangular, and as matrix
+// operands their zeros would carry a token's infinity or NaN to the tokens before it; a tile whose U is not finite
+// everywhere takes its sums over the tokens up to each one instead.
 #include "include/us_common.cuh"
 #include "include/us_f32x2.cuh"
 #include "include/us_mma.cuh"
@@ -375,6 +379,32 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) {
 // What the warps of a chunk hand on: [chunk parity][tile][half of the channels][K S0, Q S0 of eight tokens][lane],
 // accumulator tiles over that half.  In place of the first two of the other half, once they are read, U.
 using Exchange = float4[2][kTiles][kSplit][4][32];
+// entry (column, token) of two tiles [16 columns x 8 tokens] that stand side by side
+__device__ __forceinline__ float entry(const float4 (*x)[32], int col, int t) {
+  return reinterpret_cast<const float*>(&x[t >> 3][(col & 7) * 4 + ((t & 7) >> 1)])[(col >> 3) * 2 + (t & 1)];
+}
+// an FP32 value from its three parts
+__device__ __forceinline__ float whole(const unsigned char* at, int part) {
+  float sum = 0.f;
+#pragma unroll
+  for (int q = 2; q >= 0; --q) sum += us::bf2f(*reinterpret_cast<const __nv_bfloat16*>(at + q * part));
+  return sum;
+}
+// row t of M (0) or W (1) times a column, over the tokens up to t
+template <typename St>
+__device__ __forceinline__ float row_sum(const unsigned char* base, int matrix, int t, const float4 (*x)[32], int col) {
+  const unsigned char* row = base + St::kCoefs + matrix * 3 * St::kCoefPart + t * St::kCoefRow;
+  float sum = 0.f;
+#pragma unroll 1
+  for (int y = 0; y < t; ++y) sum = fmaf(whole(row + y * 2, St::kCoefPart), entry(x, col, y), sum);
+  return fmaf(reinterpret_cast<const float*>(base + St::kVec)[matrix * kChunk + t], entry(x, col, t), sum);
+}
+__device__ __forceinline__ bool all_finite(const Acc& a, const Acc& b) {
+  const f2 zero = pack2(0.f, 0.f);
+  const f2 x = fma2(b[0], zero, mul2(a[0], zero)), y = fma2(b[1], zero, mul2(a[1], zero));
+  const f2 sum = add2(x, y);
+  return !__any_sync(0xffffffffu, lo2(sum) + hi2(sum) != 0.f);
+}
 
 // The warps that feed: a chunk's vectors are on their way to registers while the one before is multiplied.
 template <int DP, bool CHANNEL>
@@ -503,19 +533,24 @@ struct Feeder {
     const float2 p = CHANNEL ? make_float2(1.f, 1.f) : *reinterpret_cast<const float2*>(vec + kChunk);
     const Acc ua = {pack2(u0.x, u0.y), pack2(u0.z, u0.w)}, ub = {pack2(u1.x, u1.y), pack2(u1.z, u1.w)};
     float o[4];
-    const Parts up(ua, ub);
-    float a1[4], a2[4];
-    mma_first(a2, up.p[0], w22[0], w22[1]);
-    mma_first(a1, up.p[0], w01[2], w01[3]);
-    mma_first(o, up.p[0], w01[0], w01[1]);
-    mma(a2, up.p[1], w01[2], w01[3]);
-    mma(a1, up.p[1], w01[0], w01[1]);
-    mma(a2, up.p[2], w01[0], w01[1]);
-    const float4 mine = half ? u1 : u0;
-    o[0] = fmaf(diag.x, mine.x, o[0] + (a1[0] + a2[0]));
-    o[1] = fmaf(diag.y, mine.y, o[1] + (a1[1] + a2[1]));
-    o[2] = fmaf(diag.x, mine.z, o[2] + (a1[2] + a2[2]));
-    o[3] = fmaf(diag.y, mine.w, o[3] + (a1[3] + a2[3]));
+    if (__builtin_expect(all_finite(ua, ub), 1)) {
+      const Parts up(ua, ub);
+      float a1[4], a2[4];
+      mma_first(a2, up.p[0], w22[0], w22[1]);
+      mma_first(a1, up.p[0], w01[2], w01[3]);
+      mma_first(o, up.p[0], w01[0], w01[1]);
+      mma(a2, up.p[1], w01[2], w01[3]);
+      mma(a1, up.p[1], w01[0], w01[1]);
+      mma(a2, up.p[2], w01[0], w01[1]);
+      const float4 mine = half ? u1 : u0;
+      o[0] = fmaf(diag.x, mine.x, o[0] + (a1[0] + a2[0]));
+      o[1] = fmaf(diag.y, mine.y, o[1] + (a1[1] + a2[1]));
+      o[2] = fmaf(diag.x, mine.z, o[2] + (a1[2] + a2[2]));
+      o[3] = fmaf(diag.y, mine.w, o[3] + (a1[3] + a2[3]));
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) o[c] = row_sum<St>(b, 1, half * 8 + 2 * i + (c & 1), u, r + (c >> 1) * 8);
+    }
     const float seen[4] = {seen0.x + seen1.x, seen0.y + seen1.y, seen0.z + seen1.z, seen0.w + seen1.w};
     const int col = col0 + tile * 16 + r;
 #pragma unroll
@@ -673,11 +708,27 @@ __global__ void __launch_bounds__(kThreads, PER_SM) chunk_delta_kernel(const Del
           u[n][c] = fma2(beta[n], w[n][c], add2(pack2(a0[n][2 * c], a0[n][2 * c + 1]), sum));
         }
     }
+    const bool finite = all_finite(u[0], u[1]);
+    auto hand_on = [&](const Acc(&z)[2]) {
 #pragma unroll
-    for (int n = 0; n < 2; ++n) other[n][lane] = make_float4(lo2(u[n][0]), hi2(u[n][0]), lo2(u[n][1]), hi2(u[n][1]));
+      for (int n = 0; n < 2; ++n) other[n][lane] = make_float4(lo2(z[n][0]), hi2(z[n][0]), lo2(z[n][1]), hi2(z[n][1]));
+    };
+    if (__builtin_expect(!finite, 0)) {               // sums over the tokens up to each one only
+      hand_on(w);
+      __syncwarp();
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int t = n * 8 + 2 * i;
+          u[n][c] = pack2(row_sum<St>(base, 0, t, other, r + c * 8), row_sum<St>(base, 0, t + 1, other, r + c * 8));
+        }
+      __syncwarp();
+    }
+    hand_on(u);
     bar_arrive(kWritesBar + (ch & 1) * (kCompute / 32) + warp, 64);
     // S' = P_16 S0 + (R K)^T U
-    {
+    if (__builtin_expect(finite, 1)) {
       // The last four tokens, which carry most of a state that decays fast, on the FP32 units: beside them the tensor
       // cores' sums would cut more of the others off.
       f2 last[kLast][2];
@@ -724,6 +775,26 @@ __global__ void __launch_bounds__(kThreads, PER_SM) chunk_delta_kernel(const Del
           }
         }
       }
+    } else {
+      __syncwarp();
+      const int n = min(kChunk, T - ch * kChunk);
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int d = dbase + 16 * j + 8 * e + 2 * i;
+            f2 sum = mul2(S[j][e][c], CHANNEL ? *reinterpret_cast<const f2*>(decay + d)
+                                              : pack2(decay[kChunk - 1], decay[kChunk - 1]));
+#pragma unroll 1
+            for (int t = 0; t < n; ++t) {
+              const unsigned char* k = base + St::kKr + t * St::kRow + d * 2;
+              const float z = entry(other, r + c * 8, t) * (CHANNEL ? 1.f : decay[kChunk + t]);
+              sum = fma2(pack2(whole(k, St::kPart), whole(k + 2, St::kPart)), pack2(z, z), sum);
+            }
+            S[j][e][c] = sum;
+          }
     }
     if (ch + 2 < chunks) bar_arrive(kEmptyBar + (ch & 1), kThreads);
   }
