@@ -68,3 +68,20 @@ def test_heads_and_gate(T, Hq, Hk, D, rot, pos0):
     assert torch.equal(v, kv[:, Hk:])
     att = torch.randn(T, Hq * D, generator=g, device="cuda").bfloat16()
     _near(HR.gate(att, proj, Hq, D), att.double() * torch.sigmoid(pairs[..., D:].reshape(T, Hq * D).double()))
+
+
+@pytest.mark.parametrize("start,stride", [(0, 64), (1, 64), (4, 64), (0, 72)])
+def test_embeddings_anywhere(start, stride):
+    """Prompt rows of a caller that start on any element, or stand apart, are served like aligned ones."""
+    from uniserve_v1_b200.models.qwen3_5 import Qwen35MoeModel
+    cfg = Qwen35MoeModel.tiny_config()
+    model = Qwen35MoeModel(cfg, "cuda", torch.bfloat16).init_random()
+    T, H = 7, cfg.hidden_size
+    buf = torch.zeros(start + T * stride, dtype=torch.bfloat16, device="cuda")
+    rows = buf[start:].view(T, stride)[:, :H]
+    rows.copy_(torch.randn(T, H, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda"))
+    ids = torch.zeros(T, dtype=torch.long)
+    got = model.forward(ids, model.new_state(), embeds=rows)
+    want = model.forward(ids, model.new_state(), embeds=rows.clone(memory_format=torch.contiguous_format))
+    # the same sums with other places of rounding to bf16, 2^-9 each, some ten a layer
+    assert float((got - want).norm() / want.norm()) < 2.0 ** -5

@@ -362,10 +362,9 @@ class Qwen35MoeModel:
         multimodal prompt (text tokens carry the same value on all three)."""
         c, w = self.cfg, self.w
         x = w["embed"][ids.to(self.device).long()] if embeds is None else \
-            embeds.to(device=self.device, dtype=self.dtype)
+            embeds.to(device=self.device, dtype=self.dtype).contiguous()
         if HR.rows_serve(x, w["norm"]):
             eps, out = c.rms_norm_eps, None
-            x = x.contiguous()
             for i in range(c.num_hidden_layers):
                 L, st = w[i], state[i]
                 x, n, _ = HR.add_norm(x, out, L["in_norm"], eps)

@@ -30,9 +30,10 @@ class Output:
 
 
 def rows_serve(x, w) -> bool:
-    """Whether ``add_norm`` takes a model of these: sixteen-byte columns of a row that a CTA holds."""
+    """Whether ``add_norm`` takes a model of these: rows in sixteen-byte columns that start on sixteen bytes, a row of
+    which a CTA holds."""
     return x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.float32 and x.dim() == 2 and \
-        x.shape[1] % 8 == 0 and x.shape[1] <= 8192
+        x.shape[1] % 8 == 0 and x.shape[1] <= 8192 and x.is_contiguous() and x.data_ptr() % 16 == 0
 
 
 def heads_serve(x, D: int) -> bool:
