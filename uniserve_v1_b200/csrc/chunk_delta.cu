@@ -813,11 +813,7 @@ __global__ void __launch_bounds__(kThreads, PER_SM) chunk_delta_kernel(const Del
 
 template <int DP, bool CHANNEL, int PER_SM>
 int launch(const DeltaRule& a, dim3 grid, int smem, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    US_CUDA_CHECK(cudaFuncSetAttribute(chunk_delta_kernel<DP, CHANNEL, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    configured = true;
-  }
+  US_CUDA_CHECK((us::allow_shared<chunk_delta_kernel<DP, CHANNEL, PER_SM>>(smem)));
   US_CUDA_CHECK(us::launch_pdl(chunk_delta_kernel<DP, CHANNEL, PER_SM>, grid, dim3(kThreads), smem, stream, a));
   return US_OK;
 }
@@ -826,12 +822,8 @@ template <int DP, bool CHANNEL>
 int launch(const DeltaRule& a, cudaStream_t stream) {
   constexpr int need = 2 * Stage<DP, CHANNEL>::kBytes;
   constexpr int alone = need > 110 * 1024 ? need : 110 * 1024;      // shared memory that one CTA per SM has
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    US_CUDA_CHECK(cudaGetDevice(&dev));
-    US_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  }
+  int sms = 0;
+  US_CUDA_CHECK(us::sm_count(&sms));
   // CTAs that are launched while the kernel before still runs would be packed two to an SM where it
   // leaves room: with fewer CTAs than SMs each asks for more shared memory than half an SM has, and may have more
   // registers (4093 rows, 32 heads of 128 x 128: 128 registers 587 us, 204 531)

@@ -10,6 +10,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "us_once.h"
+
 #define US_API extern "C" __attribute__((visibility("default")))
 
 enum UsStatus : int {
@@ -98,6 +100,24 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Lets KERNEL have `bytes` of dynamic shared memory on the current device.
+template <auto KERNEL>
+inline cudaError_t allow_shared(int bytes) {
+  static OncePerDevice once;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return (cudaError_t)once(
+      device, [&] { return (int)cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
+}
+
+// SMs of the current device.
+inline cudaError_t sm_count(int* sms) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device);
 }
 
 // CTAs a cluster of `kernel` may have: `most` (above the portable 8) where the device takes such clusters,

@@ -983,12 +983,7 @@ __global__ void __launch_bounds__(kStepThreads, 3) vector_delta_step_kernel(cons
 
 template <int LQ, int RULE>
 int launch_step(const StepArgs& a, int B, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    US_CUDA_CHECK(cudaFuncSetAttribute(vector_delta_step_kernel<LQ, RULE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kStepState));
-    configured = true;
-  }
+  US_CUDA_CHECK((us::allow_shared<vector_delta_step_kernel<LQ, RULE>>(kStepState)));
   US_CUDA_CHECK(us::launch_pdl(vector_delta_step_kernel<LQ, RULE>, dim3(a.H, B), dim3(kStepThreads),
                                (size_t)a.D * a.V * sizeof(float), stream, a));
   return US_OK;
@@ -1009,16 +1004,9 @@ template <int DP>
 int launch_rule(const RuleArgs& a, int B, cudaStream_t stream) {
   constexpr size_t need = kRuleBufs * Stage<DP>::kFloats * sizeof(float);
   constexpr size_t most = 227 * 1024;                 // shared memory of an SM's CTAs
-  static bool configured = false;
-  static int sms = 0;
-  if (!configured) {
-    int dev = 0;
-    US_CUDA_CHECK(cudaGetDevice(&dev));
-    US_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    US_CUDA_CHECK(cudaFuncSetAttribute(general_delta_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)most));
-    configured = true;
-  }
+  int sms = 0;
+  US_CUDA_CHECK(us::sm_count(&sms));
+  US_CUDA_CHECK(us::allow_shared<general_delta_kernel<DP>>((int)most));
   // CTAs that are launched while the kernel before still runs are packed where it leaves room, and the longest-running
   // SM sets the time: no SM takes more than its share of them (two sequences of 4050 tokens, 32 heads of 64 x 64: 1.69 ->
   // 1.17 ms behind a preparation that ends late).
