@@ -1,9 +1,17 @@
-"""The delta rules sixteen tokens at a time against the token by token recurrence in 64 bits, at the edges of chunks,
-tiles and widths."""
+"""The delta rules sixteen tokens at a time, and token by token where there are few, against the recurrence in 64 bits, at
+the edges of chunks, tiles and widths."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(params=["chunks", "tokens"])
+def route(request, monkeypatch):
+    """Both kernels, whatever the sizes."""
+    from uniserve_v1_b200.ops import vector_delta as VD
+    monkeypatch.setattr(VD, "few_tokens", lambda *a: request.param == "tokens")
+    return request.param
 
 
 def _inputs(lens, H, Hk, D, V, rate, per_channel):
@@ -39,7 +47,7 @@ def _recurrence(q, k, v, g, beta, S, lens, fresh):
     ([1], 2, 1, 128, 128, 0.5), ([15, 16, 17], 4, 2, 128, 128, 0.3), ([33, 1, 31], 2, 2, 64, 64, 0.05),
     ([200], 6, 3, 128, 128, 4.0), ([18, 5], 2, 1, 40, 36, 0.3), ([34], 2, 1, 256, 256, 0.1),
     ([23, 49], 2, 1, 30, 33, 0.1), ([17], 1, 1, 132, 4, 30.0), ([600], 2, 1, 128, 32, 0.001)])
-def test_chunks_follow_the_recurrence(lens, H, Hk, D, V, rate, per_channel):
+def test_chunks_follow_the_recurrence(lens, H, Hk, D, V, rate, per_channel, route):
     from uniserve_v1_b200.ops import vector_delta as VD
     q, k, v, g, beta, S = _inputs(lens, H, Hk, D, V, rate, per_channel)
     i32 = dict(dtype=torch.int32, device="cuda")
@@ -75,7 +83,7 @@ def _recurrence_fp32(q, k, v, g, beta, S):
 @pytest.mark.parametrize("per_channel", [False, True])
 @pytest.mark.parametrize("T,D,V,rate", [(16, 128, 128, 0.05), (200, 64, 64, 0.001), (500, 128, 128, 0.05),
                                          (500, 128, 128, 1.0), (300, 256, 64, 0.3), (200, 40, 36, 1.0)])
-def test_no_further_off_than_fp32(T, D, V, rate, per_channel):
+def test_no_further_off_than_fp32(T, D, V, rate, per_channel, route):
     """Operands in parts on the tensor cores against the same recurrence in FP32: as close to 64 bits (a sixth more is
     left for which values the two round differently)."""
     from uniserve_v1_b200.ops import vector_delta as VD
@@ -94,7 +102,7 @@ def test_no_further_off_than_fp32(T, D, V, rate, per_channel):
 @pytest.mark.parametrize("per_channel", [False, True])
 @pytest.mark.parametrize("where", ["v", "k", "q", "g"])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
-def test_not_finite_stays_with_later_tokens(where, bad, per_channel):
+def test_not_finite_stays_with_later_tokens(where, bad, per_channel, route):
     """A token that is not finite in the middle of a chunk: tokens before it, and for a value the other columns, are what
     they are without it."""
     from uniserve_v1_b200.ops import vector_delta as VD
@@ -123,3 +131,27 @@ def test_not_finite_stays_with_later_tokens(where, bad, per_channel):
         assert not bool(torch.isfinite(got[at, head]).any())
     else:
         assert not bool(torch.isfinite(got[at:, head]).any())
+
+
+@pytest.mark.parametrize("lens,H,D,per_channel,names", [
+    ([48], 32, 128, False, ["us_token_delta_rule"]), ([49], 32, 128, False, ["us_head_delta_rule"]),
+    ([1] * 7, 4, 64, True, ["us_token_delta_rule"]), ([65], 4, 64, True, ["us_channel_delta_rule"]),
+    ([1] * 63 + [200], 2, 128, True, ["us_channel_delta_rule"]), ([80] * 3, 128, 64, True, ["us_token_delta_rule"])])
+def test_route(lens, H, D, per_channel, names, monkeypatch):
+    """Which kernel runs, with the lengths on the host and, from the number of rows alone, without."""
+    from uniserve_v1_b200.ops import native as N
+    from uniserve_v1_b200.ops import vector_delta as VD
+    q, k, v, g, beta, S = _inputs(lens, H, H, D, D, 0.3, per_channel)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], **i32)
+    pos = torch.cat([torch.arange(n, **i32) + 7 for n in lens])
+    m = VD.SeqMeta(cu, torch.arange(len(lens), **i32), pos, False, [7] * len(lens), lens)
+    called, call = [], N.call
+    monkeypatch.setattr(N, "call", lambda name, *a, **kw: (called.append(name), call(name, *a, **kw))[1])
+    S0 = S.clone()
+    out = VD.vector_delta_rule(q, k, v, g, S, m, beta=beta)
+    assert called == names
+    bare = VD.SeqMeta(cu, m.slots, pos, False)
+    again = VD.vector_delta_rule(q, k, v, g, S0, bare, beta=beta)
+    # two kernels, each within the bound above of 64 bits
+    assert float((out - again).norm() / out.norm()) < 1e-6 and float((S - S0).norm() / S.norm()) < 1e-6

@@ -11,7 +11,8 @@
 //                           g = exp(-exp(A_log) softplus(low + dt_bias)) and beta = sigmoid(b)
 //   us_head_delta_prep      the same with the decay's argument a column per head of the projection
 //   us_general_delta_prep   decay w = exp(-c sigmoid(low + w0)), unit key n, removal a * n
-//   us_general_delta_rule   the general recurrence (the two others': chunk_delta.cu)
+//   us_general_delta_rule   the general recurrence, us_token_delta_rule the two others for a few tokens of every
+//                           sequence (chunk_delta.cu: for more)
 //   us_head_norm_gate       per-head RMS norm of o, weight, sigmoid or silu gate
 //   us_{channel,head,general}_delta_step   all of these for one token of every sequence in one launch
 //
@@ -20,7 +21,7 @@
 // starts from a zero state whatever its slot holds: slots are handed on without being cleared,
 // and nothing has to be launched when a request is admitted.  A negative slot marks padding.
 //
-// General rule kernel: a CTA owns 32 value columns of one head of one sequence.  A lane holds D/8 rows x 2
+// Rule kernel: a CTA owns 32 value columns of one head of one sequence.  A lane holds D/8 rows x 2
 // columns of S in registers as row pairs (packed FP32 instructions), so the two D-long reductions
 // of a token are short chains and three shuffles; the read-out's is folded beside the next token's
 // first one.  A token depends on the one before through one reduction and one update: that chain
@@ -453,9 +454,10 @@ constexpr int kRuleBufs = 4;                         // chunks of vectors in sha
 
 struct RuleArgs {
   const float *q, *k, *v;         // [rows, Hk, D] x 2, [rows, H, V]
-  const float* g;                 // decay [rows, H, D]
-  const float* n;                 // removal direction [rows, H, D]
-  const float* p;                 // removal rate * direction [rows, H, D]
+  const float* g;                 // decay [rows, H, D], head: [rows, H]
+  const float* n;                 // general: removal direction [rows, H, D]
+  const float* p;                 // general: removal rate * direction [rows, H, D]
+  const float* beta;              // channel, head: [rows, H]
   float* state;                   // [slots, H, D, V]
   float* out;                     // [rows, H, V]
   const int *cu, *slots, *pos;
@@ -478,11 +480,14 @@ __device__ __forceinline__ void cp_async(float* dst, const float* src) {
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-// A token in shared memory: kVecs vectors of DP floats (g, k, q, n, p), then 32 columns of v.
-template <int DP>
+// A token in shared memory: vectors of DP floats (g but for the head rule, k, q and, general, n, p), then 32 columns of
+// v, beta and the head rule's g.
+template <int DP, int RULE>
 struct Stage {
-  static constexpr int kVecs = 5;
-  static constexpr int kToken = kVecs * DP + kCols + 4;
+  static constexpr int kFirst = RULE == kHead ? 1 : 0;            // vectors are numbered g, k, q, n, p
+  static constexpr int kVecs = RULE == kGeneral ? 5 : 3 - kFirst;
+  static constexpr int kK = (1 - kFirst) * DP, kQ = kK + DP, kN = kQ + DP, kP = kN + DP, kV = kVecs * DP, kBeta = kV + kCols;
+  static constexpr int kToken = kV + kCols + 4;
   static constexpr int kChunk = 8;                    // tokens per chunk
   static constexpr int kFloats = kChunk * kToken;
 };
@@ -490,18 +495,22 @@ struct Stage {
 // Asynchronous copies of tokens' vectors by the copying threads.  Widths that are multiples of
 // four move as 16-byte pieces: a thread owns the same pieces of every token and only advances its
 // pointers (address arithmetic per piece would cost as much as the recurrence).
-template <int DP>
+template <int DP, int RULE>
 struct Copier {
-  using St = Stage<DP>;
+  using St = Stage<DP, RULE>;
   static constexpr int kQ = DP / 4;
   static constexpr int kPieces = St::kVecs * kQ + kCols / 4;
   static constexpr int kMine = (kPieces + kRuleCopy - 1) / kRuleCopy;
   const float* src[kMine];
   int step[kMine], dst[kMine];          // floats per token, place in the token (-1: nothing)
-  int tid;
+  const float *beta, *decay;            // numbers of a token
+  int tid, heads;
   bool quad;
   __device__ __forceinline__ void init(const RuleArgs& a, int tid_, long long row0, int h, int hk, int col0) {
     tid = tid_;
+    heads = a.H;
+    beta = RULE == kGeneral ? nullptr : a.beta + row0 * a.H + h;
+    decay = RULE == kHead ? a.g + row0 * a.H + h : nullptr;
     quad = (a.V & 3) == 0 && (a.D & 3) == 0;
 #pragma unroll
     for (int i = 0; i < kMine; ++i) {
@@ -511,9 +520,10 @@ struct Copier {
       step[i] = 0;
       if (e < St::kVecs * kQ) {
         if (d >= a.D) continue;
-        const bool shared = vec == 1 || vec == 2;
+        const int id = vec + St::kFirst;
+        const bool shared = id == 1 || id == 2;
         const int heads_ = shared ? a.Hk : a.H, hh = shared ? hk : h;
-        src[i] = (vec == 1 ? a.k : vec == 2 ? a.q : vec == 0 ? a.g : vec == 3 ? a.n : a.p) +
+        src[i] = (id == 1 ? a.k : id == 2 ? a.q : id == 0 ? a.g : id == 3 ? a.n : a.p) +
                  (row0 * heads_ + hh) * a.D + d;
         step[i] = heads_ * a.D;
         dst[i] = vec * DP + d;
@@ -537,27 +547,38 @@ struct Copier {
             cp_async<16>(buf + dst[i], src[i]);
             src[i] += step[i];
           }
+        numbers(buf);
       }
     } else {
       for (int t = 0; t < n; ++t, buf += St::kToken) {
         const long long row = row0 + t;
         for (int e = tid; e < St::kVecs * a.D; e += kRuleCopy) {
-          const int vec = e / a.D, d = e - vec * a.D;
-          const bool shared = vec == 1 || vec == 2;
-          const float* from = vec == 1 ? a.k : vec == 2 ? a.q : vec == 0 ? a.g : vec == 3 ? a.n : a.p;
+          const int vec = e / a.D, d = e - vec * a.D, id = vec + St::kFirst;
+          const bool shared = id == 1 || id == 2;
+          const float* from = id == 1 ? a.k : id == 2 ? a.q : id == 0 ? a.g : id == 3 ? a.n : a.p;
           cp_async<4>(buf + vec * DP + d, from + (shared ? row * a.Hk + hk : row * a.H + h) * a.D + d);
         }
         for (int c = tid; c < kCols && col0 + c < a.V; c += kRuleCopy)
           cp_async<4>(buf + St::kVecs * DP + c, a.v + (row * a.H + h) * a.V + col0 + c);
+        numbers(buf);
       }
+    }
+  }
+  __device__ __forceinline__ void numbers(float* buf) {
+    if (RULE == kGeneral || tid != 0) return;
+    cp_async<4>(buf + St::kBeta, beta);
+    beta += heads;
+    if (RULE == kHead) {
+      cp_async<4>(buf + St::kBeta + 1, decay);
+      decay += heads;
     }
   }
 };
 
-template <int DP>
-__global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) general_delta_kernel(const RuleArgs a) {
+template <int DP, int RULE>
+__global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) token_delta_kernel(const RuleArgs a) {
   US_PDL_PROLOGUE();
-  using St = Stage<DP>;
+  using St = Stage<DP, RULE>;
   constexpr int NG = DP / 32;                         // groups of four rows per lane
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -579,7 +600,7 @@ __global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) general_delta_
     __syncthreads();
   }
   if (tid >= kRuleCompute) {                          // the copying threads stay one chunk ahead
-    Copier<DP> cp;
+    Copier<DP, RULE> cp;
     cp.init(a, tid - kRuleCompute, start, h, hk, col0);
     const int chunks = (T + St::kChunk - 1) / St::kChunk;
     auto fetch = [&](int r) {                         // (an empty group past the end)
@@ -641,13 +662,23 @@ __global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) general_delta_
     __syncthreads();                                  // this chunk's vectors are there
     const float* base = sm + buf * St::kFloats;
     for (int t = 0; t < n; ++t, base += St::kToken) {
-      const float* vs = base + St::kVecs * DP;
+      const float* vs = base + St::kV;
+      const f2 decay = RULE == kHead ? pack2(vs[kCols + 1], vs[kCols + 1]) : 0ull;
       f2 y[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
 #pragma unroll
       for (int j = 0; j < NG; ++j) {
         const int r0 = (j * 8 + kq) * 4;
         f2 m[2];
-        lds_vec(m, base + 3 * DP + r0);
+        lds_vec(m, base + (RULE == kGeneral ? St::kN : St::kK) + r0);
+        if (RULE != kGeneral) {
+          f2 g[2] = {decay, decay};
+          if (RULE == kChannel) lds_vec(g, base + r0);
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int c = 0; c < 2; ++c)     // the key sees the decayed state
+              S[j * 2 + e][c] = mul2(S[j * 2 + e][c], g[e]);
+        }
 #pragma unroll
         for (int e = 0; e < 2; ++e)
 #pragma unroll
@@ -662,25 +693,34 @@ __global__ void __launch_bounds__(kRuleThreads, DP > 128 ? 1 : 3) general_delta_
         op += ostep;
       }
       pending = true;
-      const float other = __shfl_xor_sync(0xffffffffu, seen, 4);     // n^T S of this lane's column
-      const float u0 = up ? other : seen, u1 = up ? seen : other;
-      const float2 v2 = *reinterpret_cast<const float2*>(vs + cb);
-      const f2 uu[2] = {pack2(-u0, -u0), pack2(-u1, -u1)}, vv[2] = {pack2(v2.x, v2.x), pack2(v2.y, v2.y)};
+      float c = seen;                               // general: n^T S of this lane's column
+      if (RULE != kGeneral) c = vs[kCols] * (vs[cb + (up ? 1 : 0)] - seen);
+      const float other = __shfl_xor_sync(0xffffffffu, c, 4);
+      const float u0 = up ? other : c, u1 = up ? c : other;
+      f2 uu[2] = {pack2(u0, u0), pack2(u1, u1)}, vv[2];
+      if (RULE == kGeneral) {
+        const float2 v2 = *reinterpret_cast<const float2*>(vs + cb);
+        uu[0] = pack2(-u0, -u0); uu[1] = pack2(-u1, -u1);
+        vv[0] = pack2(v2.x, v2.x); vv[1] = pack2(v2.y, v2.y);
+      }
       f2 oo[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
 #pragma unroll
       for (int j = 0; j < NG; ++j) {
         const int r0 = (j * 8 + kq) * 4;
         f2 k[2], q[2], g[2], p[2];
-        lds_vec(k, base + DP + r0);
-        lds_vec(q, base + 2 * DP + r0);
-        lds_vec(g, base + r0);
-        lds_vec(p, base + 4 * DP + r0);
+        lds_vec(k, base + St::kK + r0);
+        lds_vec(q, base + St::kQ + r0);
+        if (RULE == kGeneral) {
+          lds_vec(g, base + r0);
+          lds_vec(p, base + St::kP + r0);
+        }
 #pragma unroll
         for (int e = 0; e < 2; ++e)
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             f2& x = S[j * 2 + e][c];
-            x = fma2(k[e], vv[c], fma2(p[e], uu[c], mul2(g[e], x)));
+            if (RULE == kGeneral) x = fma2(k[e], vv[c], fma2(p[e], uu[c], mul2(g[e], x)));
+            else x = fma2(k[e], uu[c], x);
             oo[c][e] = fma2(x, q[e], oo[c][e]);
           }
       }
@@ -1000,13 +1040,13 @@ int step_impl(StepArgs a, int B, cudaStream_t stream) {
   return launch_step<64, RULE>(a, B, stream);
 }
 
-template <int DP>
+template <int DP, int RULE>
 int launch_rule(const RuleArgs& a, int B, cudaStream_t stream) {
-  constexpr size_t need = kRuleBufs * Stage<DP>::kFloats * sizeof(float);
+  constexpr size_t need = kRuleBufs * Stage<DP, RULE>::kFloats * sizeof(float);
   constexpr size_t most = 227 * 1024;                 // shared memory of an SM's CTAs
   int sms = 0;
   US_CUDA_CHECK(us::sm_count(&sms));
-  US_CUDA_CHECK(us::allow_shared<general_delta_kernel<DP>>((int)most));
+  US_CUDA_CHECK((us::allow_shared<token_delta_kernel<DP, RULE>>((int)most)));
   // CTAs that are launched while the kernel before still runs are packed where it leaves room, and the longest-running
   // SM sets the time: no SM takes more than its share of them (two sequences of 4050 tokens, 32 heads of 64 x 64: 1.69 ->
   // 1.17 ms behind a preparation that ends late).
@@ -1014,8 +1054,21 @@ int launch_rule(const RuleArgs& a, int B, cudaStream_t stream) {
   const size_t share = ((size_t)grid.x * grid.y * grid.z + sms - 1) / sms;
   size_t smem = most / (share + 1) + 1024;
   if (smem < need || share > 4) smem = need;
-  US_CUDA_CHECK(us::launch_pdl(general_delta_kernel<DP>, grid, dim3(kRuleThreads), smem, stream, a));
+  US_CUDA_CHECK(us::launch_pdl(token_delta_kernel<DP, RULE>, grid, dim3(kRuleThreads), smem, stream, a));
   return US_OK;
+}
+
+template <int RULE>
+int rule_impl(const RuleArgs& a, int B, cudaStream_t stream) {
+  US_REQUIRE(a.q && a.k && a.v && a.g && a.state && a.out && a.cu && a.slots && a.pos && B >= 1 && B <= 65535);
+  US_REQUIRE(a.H >= 1 && a.Hk >= 1 && a.H % a.Hk == 0 && a.H <= 65535 && a.D >= 1 && a.V >= 1);
+  US_REQUIRE((a.D & 3) || (a.V & 3) || (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (RULE == kHead ? 0 : (uintptr_t)a.g) |
+               (uintptr_t)a.n | (uintptr_t)a.p | (uintptr_t)a.state) % 16) == 0);
+  if (a.D <= 32) return launch_rule<32, RULE>(a, B, stream);
+  if (a.D <= 64) return launch_rule<64, RULE>(a, B, stream);
+  if (a.D <= 128) return launch_rule<128, RULE>(a, B, stream);
+  if (a.D <= 256) return launch_rule<256, RULE>(a, B, stream);
+  return US_ERR_UNSUPPORTED;
 }
 
 int prep_impl(const ChannelPrep& a, cudaStream_t stream) {
@@ -1119,22 +1172,22 @@ US_API int us_general_delta_prep(const void* x, long long ldx, int off_r, int of
   return US_OK;
 }
 
-// general = 0: the channel rule (g, beta); 1: the general rule (g, n, p).  q and k heads serve
-// H / Hk value heads each; all vectors dense FP32.
+// q and k heads serve H / Hk value heads each; all vectors dense FP32.
 US_API int us_general_delta_rule(const float* q, const float* k, const float* v, const float* g, const float* n,
                                  const float* p, float* state, float* out, const int* cu, const int* slots,
                                  const int* pos, int B, int H, int Hk, int D, int V, void* stream_) {
-  US_REQUIRE(q && k && v && g && n && p && state && out && cu && slots && pos && B >= 1 && B <= 65535);
-  US_REQUIRE(H >= 1 && Hk >= 1 && H % Hk == 0 && H <= 65535 && D >= 1 && V >= 1);
-  US_REQUIRE((D & 3) || (V & 3) || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)g | (uintptr_t)n |
-               (uintptr_t)p | (uintptr_t)state) % 16) == 0);
-  RuleArgs a{q, k, v, g, n, p, state, out, cu, slots, pos, H, Hk, D, V};
-  cudaStream_t stream = (cudaStream_t)stream_;
-  if (D <= 32) return launch_rule<32>(a, B, stream);
-  if (D <= 64) return launch_rule<64>(a, B, stream);
-  if (D <= 128) return launch_rule<128>(a, B, stream);
-  if (D <= 256) return launch_rule<256>(a, B, stream);
-  return US_ERR_UNSUPPORTED;
+  US_REQUIRE(n && p);
+  return rule_impl<kGeneral>(RuleArgs{q, k, v, g, n, p, nullptr, state, out, cu, slots, pos, H, Hk, D, V}, B,
+                             (cudaStream_t)stream_);
+}
+
+// The channel rule (g [rows, H, D]) or the head rule (g [rows, H]) for sequences of few tokens.
+US_API int us_token_delta_rule(int per_channel, const float* q, const float* k, const float* v, const float* g,
+                               const float* beta, float* state, float* out, const int* cu, const int* slots,
+                               const int* pos, int B, int H, int Hk, int D, int V, void* stream_) {
+  US_REQUIRE(beta);
+  const RuleArgs a{q, k, v, g, nullptr, nullptr, beta, state, out, cu, slots, pos, H, Hk, D, V};
+  return per_channel ? rule_impl<kChannel>(a, B, (cudaStream_t)stream_) : rule_impl<kHead>(a, B, (cudaStream_t)stream_);
 }
 
 US_API int us_head_norm_gate(const float* o, const float* w, int w_head_stride, const void* gate,

@@ -366,7 +366,7 @@ class NepevikModel(LayeredDecoder):
         """Final-normed rows [T, Wp] of the packed batch ``meta`` (``cu_q``, ``state_slots``,
         ``page_table``, ``slots``); ``meta.states`` are the pools of ``new_state_pools``."""
         c = self.cfg
-        m = VD.SeqMeta(meta.cu_q, meta.state_slots, positions, meta.kind == "decode")
+        m = VD.SeqMeta(meta.cu_q, meta.state_slots, positions, meta.kind == "decode", meta.context_lens, meta.q_lens)
         res, x = F.embed_rows(input_ids, self.embed)
         routes: dict = {}
         for tables, of in self.tables:

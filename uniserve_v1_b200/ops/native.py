@@ -48,6 +48,7 @@ _SIGNATURES = {
                                   I, I, I, I, I, I, I, I, I, P]),
     "us_general_delta_prep": (I, [P, L, I, I, I, I, P, L, P, P, P, I, I, I, F, I, P]),
     "us_general_delta_rule": (I, [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]),
+    "us_token_delta_rule": (I, [I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]),
     "us_channel_delta_step": (I, [P, L, I, I, I, I, P, P, P, P, L, P, P, P, P, P, I, P, L, P, L, P, P,
                                   I, I, I, I, I, I, F, I, I, P]),
     "us_general_delta_step": (I, [P, L, I, I, I, I, P, L, P, P, P, P, I, P, L, P, L, P, P, I, I, I, F,

@@ -8,7 +8,7 @@ per head.
 Batches are packed: rows of sequence s are cu[s] .. cu[s + 1], its state lives in slot
 ``slots[s]`` of a pool and is updated in place; a sequence whose first row stands at position 0
 starts from zero whatever the slot holds, a negative slot marks padding.  On a GPU the entry
-points run ``csrc/vector_delta.cu`` (the channel and head rules' recurrences: ``csrc/chunk_delta.cu``); on the CPU the same recurrences run step by step in FP32.
+points run ``csrc/vector_delta.cu`` (the channel and head rules of more than a few tokens: ``csrc/chunk_delta.cu``); on the CPU the same recurrences run step by step in FP32.
 """
 from __future__ import annotations
 
@@ -151,6 +151,19 @@ def general_prep(x, offs, low, w, H, D):
     return torch.exp(-GENERAL_DECAY_RATE * torch.sigmoid(low + w["w0"])).view(T, H, D), n, a * n, k, r, v
 
 
+def few_tokens(rows: int, longest: int, H: int, D: int, per_channel: bool) -> bool:
+    """Whether the channel and head rules go token by token (``us_token_delta_rule``) rather than in chunks of sixteen:
+    a chunk costs the same for one token as for sixteen, and its coefficients a launch.  Measured with 32 heads (us, a
+    decay per head, chunks / tokens).  128 wide: one sequence of 16 tokens 16 / 10, 48 21 / 18, 96 28 / 29; 8 sequences of
+    16 37 / 33, 48 60 / 62; 64 sequences of one 170 / 158, of 4 174 / 177, of 16 189 / 251, since with the chip full the
+    products' number counts and not their chain.  64 wide: 64 sequences of one 60 / 27, of 16 65 / 56, of 64 170 / 166,
+    one of 96 18 / 19.  A decay per channel, 64 wide, costs a chunk more: 64 sequences of 64 250 / 176, 8 of 500 238 / 180
+    with the chip full, one of 4093 473 / 685 where the longest chain sets the time."""
+    if D > 64:
+        return longest <= 48 and rows * H <= 12288
+    return longest <= 64 or (per_channel and rows * H >= 256 * longest)
+
+
 def vector_delta_rule(q, k, v, g, state, m: SeqMeta, beta=None, n=None, p=None):
     """The recurrence.  q, k [T, Hk, D], v [T, H, V], g / n / p [T, H, D] and beta [T, H] are dense
     FP32; ``beta`` selects the channel rule (with g [T, H] the head rule), ``n`` and ``p`` the general
@@ -162,6 +175,11 @@ def vector_delta_rule(q, k, v, g, state, m: SeqMeta, beta=None, n=None, p=None):
         for t in (q, k, v, g, state):
             assert t.dtype == torch.float32 and t.is_contiguous()
         out = torch.empty(T, H, V, dtype=torch.float32, device=q.device)
+        if not general and few_tokens(T, max(m.lengths) if m.lengths else T, H, D, g.dim() == 3):
+            N.call("us_token_delta_rule", int(g.dim() == 3), N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(g), N.ptr(beta),
+                   N.ptr(state), N.ptr(out), N.ptr(m.cu), N.ptr(m.slots), N.ptr(m.positions), m.slots.shape[0], H, Hk, D,
+                   V, N.stream())
+            return out
         if not general:
             coef = torch.empty(N.kernels().us_delta_coef_floats(T, m.slots.shape[0], H), dtype=torch.float32,
                                device=q.device)
