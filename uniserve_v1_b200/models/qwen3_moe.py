@@ -486,7 +486,7 @@ class Qwen3MoeModel:
             return x, ("ep", ids)
         ws = None
         if x.is_cuda:
-            key = (T, x.device)
+            key = (T, x.device, lw.fp8 is not None)
             ws = self._moe_ws.get(key)
             if ws is None:
                 ws = F.MoeWorkspace.create(T, cfg.num_experts_per_tok, self.E_local,
@@ -519,10 +519,6 @@ class Qwen3MoeModel:
         self._count_experts(lw, ids, getattr(self, "_live", None) if fused_route else None)
         if lw.fp8 is not None:
             from ..ops.fp8 import moe_experts_fp8
-            if ws is not None and ws.block_n > 64:
-                ws = self._moe_ws[key] = F.MoeWorkspace.create(
-                    T, cfg.num_experts_per_tok, self.E_local, cfg.hidden_size,
-                    cfg.moe_intermediate_size, x.device, fp8=True)
             out = moe_experts_fp8(x, ids, weights, lw.fp8, e_lo=self.e_lo, ws=ws)
         else:
             later = defer and small and FUSED_UNPERMUTE and (fc is not None or not reduce)

@@ -450,19 +450,32 @@ def topk_softmax(logits, top_k, renorm=True, live=None, expert_map=None, load=No
 MOE_PAIR_MIN_ROWS = int(_os.environ.get("US_MOE_PAIR_ROWS", "96"))
 
 
-def _tile_rows(per: float, gated: bool = True, fp8: bool = False) -> int:
-    """Rows per tile for ``per`` routes to an expert on average (single-CTA kernels).  A tile streams its expert's
-    weights, so two tiles of an expert cost up to twice one; a wider one multiplies more empty rows and holds fewer
-    stages.  Measured at 128 experts of 2048 x 768 and 4096 x 1536 and 64 of 2048 x 768 (us of a whole layer, rows per
-    tile 16 / 32 / 64, CTA pairs of 256): 13 routes 229 / 219 / 252 / 431, 25 routes 273 / 233 / 285 / 435, 56 routes 425 / 316 /
-    343 / 452, 75 routes - / 370 / 456 / 449, 113 routes - / 474 / 551 / 456; below 4 routes 16 and 32 change places within 3 %.
-    FP8: 6 routes 164 / 169, 16 routes 607 / 532 / 780, 56 routes 461 / 385 / 597.  Ungated (64 experts of 2048 x 1024): 4 routes
-    95 / 96 / 96, 16 routes 109 / 104 / 104, 32 routes 139 / 127 / 115, 64 routes 185 / 155 / 146 / 161, 94 routes 249 / 194 / 167 / 163."""
+def _tile_rows(per: float, experts: int, gated: bool = True, fp8: bool = False) -> int:
+    """Rows per tile for ``per`` routes to each of ``experts`` on average (single-CTA kernels).  A tile streams its
+    expert's weights, so two tiles of an expert cost up to twice one; a wider one multiplies more empty rows and holds
+    fewer stages.  Measured in us of a whole layer, rows per tile 16 / 32 / 64 (/ CTA pairs of 256).
+
+    Gated bf16, 128 experts of 2048 x 768: 1 route 135 / 158, 2 189 / 188, 4 208 / 208, 8 213 / 213, 13 216 / 221, 25 273 / 233 /
+    285 / 435, 56 425 / 316 / 343 / 452, 75 - / 370 / 456 / 449, 113 - / 474 / 551 / 456.  64 of them: 1 86 / 90, 2 116 / 104, 4 121 / 115,
+    8 127 / 117, 13 127 / 121.  128 of 4096 x 1536: 1 477 / 495, 2 620 / 631, 4 726 / 726, 8 744 / 740, 13 779 / 764.
+    FP8, 128 of 2048 x 768: 8 165 / 186 / 261, 13 197 / 183 / 272, 25 259 / 227 / 350, 128 899 / 718 / 1181, 510 3377 / 2624 / 4334.
+    64 of them: 10 106 / 118 / 151, 16 115 / 128 / 167, 25 144 / 149 / 208, 40 189 / 183 / 267, 510 1706 / 1338 / 2191.  128 of 4096 x 1536:
+    8 482 / 479 / 695, 13 525 / 514 / 738, 25 697 / 613 / 934, 510 9931 / 7466 / 12483: where 16 and 32 change places goes with
+    the routes in all.  Ungated (64 experts of 2048 x 1024): 4 95 / 96 / 96, 16 109 / 104 / 104, 32 139 / 127 / 115, 64 185 / 155 /
+    146 / 161, 94 249 / 194 / 167 / 163."""
     if fp8:
         return 16 if per <= 10 else 32
     if gated:
         return 16 if per < 4 else 32 if per < 96 else 128
     return 16 if per < 12 else 32 if per < 24 else 64 if per < 96 else 128
+
+
+def _block_rows(R_: int, E: int, E_total: int, gated: bool = True, fp8: bool = False) -> int:
+    """Rows per tile of R_ routes over E_total experts, E of them here."""
+    # prefill-size batches (a few hundred rows per expert): 256-row tiles on CTA pairs
+    if not fp8 and R_ // max(1, E_total) >= MOE_PAIR_MIN_ROWS:
+        return 256
+    return _tile_rows(R_ / max(1, E_total), E, gated, fp8)
 
 
 @dataclass
@@ -489,10 +502,7 @@ class MoeWorkspace:
         them (the routes then spread over all ranks; sizes the expected live tiles)."""
         R_ = T * top_k
         if block_n is None:
-            block_n = _tile_rows(R_ / max(1, E_local), fp8=fp8)
-            # prefill-size batches (a few hundred rows per expert): 256-row tiles on CTA pairs
-            if not fp8 and R_ // max(1, E_total or E_local) >= MOE_PAIR_MIN_ROWS:
-                block_n = 256
+            block_n = _block_rows(R_, E_local, E_total or E_local, fp8=fp8)
         max_tiles = min(R_, E_local) + R_ // block_n + 1
         i32 = dict(dtype=torch.int32, device=device)
         return MoeWorkspace(
@@ -658,9 +668,7 @@ class Routes:
 
 def _route_tiles(R_, E, E_total, gated=True):
     """(rows per tile, most tiles, expected live tiles) of R_ routes over E_total experts, E of them here."""
-    block_n = _tile_rows(R_ / E_total, gated)
-    if R_ // E_total >= MOE_PAIR_MIN_ROWS:
-        block_n = 256
+    block_n = _block_rows(R_, E, E_total, gated)
     return block_n, min(R_, E) + R_ // block_n + 1, MoeWorkspace._expected_tiles(R_, E, E_total, block_n)
 
 

@@ -87,19 +87,17 @@ class ExpertExchange:
         self.recv_ptrs = (ctypes.c_void_p * world)(*[lib.us_ep_peer_recv(self.h, r) for r in range(world)])
         self._ws = {}
 
-    def workspace(self, t_step: int):
+    def workspace(self, t_step: int, fp8: bool = False):
         """Sort / GEMM workspace for a step of ``t_step`` rows per source (the window
         stride of that step; the same on every rank, which run in lock step)."""
-        ws = self._ws.get(t_step)
+        ws = self._ws.get((t_step, fp8))
         if ws is None:
-            ws = F.MoeWorkspace.create(self.world * t_step, self.k, self.experts_per_rank, self.H,
-                                       self.I, self.device)
-            if ws.block_n > 128:
-                # FC2 pushes its rows to the token owners from the single-CTA grouped kernel's
-                # epilogue: 128-row tiles (the 256-row tiles belong to the CTA-pair kernel)
-                ws = F.MoeWorkspace.create(self.world * t_step, self.k, self.experts_per_rank,
-                                           self.H, self.I, self.device, block_n=128)
-            self._ws[t_step] = ws
+            # FC2 pushes its rows to the token owners from the single-CTA grouped kernel's
+            # epilogue: at most 128-row tiles (the 256-row tiles belong to the CTA-pair kernel)
+            rows = F._block_rows(self.world * t_step * self.k, self.experts_per_rank, self.E, fp8=fp8)
+            ws = self._ws[t_step, fp8] = F.MoeWorkspace.create(
+                self.world * t_step, self.k, self.experts_per_rank, self.H, self.I, self.device,
+                block_n=min(rows, 128), E_total=self.E)
         return ws
 
     def close(self):
@@ -153,11 +151,7 @@ class ExpertExchange:
         that arrived are quantised per row and 128-wide K block before each grouped
         GEMM; FC2's epilogue pushes the weighted rows to the token owners."""
         from ..ops import fp8 as Q
-        ws, st = self.workspace(t_step), N.stream()
-        if ws.block_n > 64:
-            ws = self._ws[t_step] = F.MoeWorkspace.create(
-                self.world * t_step, self.k, self.experts_per_rank, self.H, self.I, self.device,
-                block_n=64)
+        ws, st = self.workspace(t_step, fp8=True), N.stream()
         E, I2, H = ex.w13.shape
         I_ = I2 // 2
         R = self.world * t_step * self.k

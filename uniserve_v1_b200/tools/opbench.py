@@ -213,9 +213,7 @@ def main():
         ex = Q.Fp8Experts.from_bf16(rnd(E, 2 * I, H), rnd(E, H, I))
         logits = torch.randn(T, E, generator=g, device=dev)
         ids, wts = F.topk_softmax(logits, k, True)
-        ws = F.MoeWorkspace.create(T, k, E, H, I, dev)
-        if ws.block_n > 64:
-            ws = F.MoeWorkspace.create(T, k, E, H, I, dev, block_n=64)
+        ws = F.MoeWorkspace.create(T, k, E, H, I, dev, fp8=True)
         ms = timeit(lambda: Q.moe_experts_fp8(x, ids, wts, ex, ws=ws), a.iters)
         active = int(torch.unique(ids).numel())
         byts = active * (ex.w13[0].numel() + ex.w2[0].numel()) * 1.0
