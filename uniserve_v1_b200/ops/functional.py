@@ -464,7 +464,7 @@ def _tile_rows(per: float, experts: int, gated: bool = True, fp8: bool = False) 
     the routes in all.  Ungated (64 experts of 2048 x 1024): 4 95 / 96 / 96, 16 109 / 104 / 104, 32 139 / 127 / 115, 64 185 / 155 /
     146 / 161, 94 249 / 194 / 167 / 163."""
     if fp8:
-        return 16 if per <= 10 else 32
+        return 16 if per * experts <= 1280 else 32
     if gated:
         return 16 if per < 4 else 32 if per < 96 else 128
     return 16 if per < 12 else 32 if per < 24 else 64 if per < 96 else 128
