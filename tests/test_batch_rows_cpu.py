@@ -57,3 +57,17 @@ def test_pages_that_do_not_hold_the_tokens(held, most, bad):
     plan = array("i", start + length + [len(p) for p in pages] + [0, 1] + [x for p in pages for x in p])
     rc, _ = _run(plan, list(range(25)), 2, 25, 16, most, 90, 200)
     assert rc == bad
+
+
+@pytest.mark.parametrize("pages,why", [([1, 2, 3], "3 pages, a row of the page table takes 2"),
+                                        ([1], "its pages do not hold its tokens")])
+def test_refusal_names_its_reason(pages, why):
+    from types import SimpleNamespace
+
+    import torch
+
+    from uniserve_v1_b200.engine.runner import CausalLmRunner
+    runner = SimpleNamespace(device=torch.device("cpu"), attends_pages=True, max_pages=2, page_size=4)
+    request = SimpleNamespace(token_slice=lambda a, b: [7] * (b - a), pages=pages, slot=0, request_id="r")
+    with pytest.raises(IndexError, match=f"request r: {why}"):
+        CausalLmRunner._prefill_rows(runner, [SimpleNamespace(start=0, length=6, request=request)])

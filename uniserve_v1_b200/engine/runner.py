@@ -743,7 +743,10 @@ class CausalLmRunner:
         bad = N.host().us_batch_rows(*(ctypes.c_void_p(x.buffer_info()[0]) for x in (plan, ids)), B, T,
                                      self.page_size, self.max_pages if tables else 0, first, N.ptr(packed))
         if bad:
-            raise IndexError(f"request {chunks[bad - 1].request.request_id}: its pages do not hold its tokens")
+            req = chunks[bad - 1].request
+            why = (f"{len(req.pages)} pages, a row of the page table takes {self.max_pages}"
+                   if tables and len(req.pages) > self.max_pages else "its pages do not hold its tokens")
+            raise IndexError(f"request {req.request_id}: {why}")
         d = packed.to(dev, non_blocking=True)
         self.h2d_bytes += packed.numel() * 4
         page_table = d[first:].view(B, self.max_pages) if tables else None
