@@ -786,7 +786,7 @@ def test_gated_delta_rule_kernel(Dk, Dv, Hk, Hv, dtype):
 @pytest.mark.parametrize("Dk,Dv,Hk,Hv,K,lens,dtype", [
     (128, 128, 2, 4, 4, [16, 67], BF), (36, 20, 2, 2, 2, [131], torch.float32), (64, 132, 1, 3, 3, [2, 33, 13], BF)])
 def test_hybrid_mixer_rows(Dk, Dv, Hk, Hv, K, lens, dtype):
-    """Preparation and four-token recurrence of the hybrid layers' prompts (fewer rows than taps, blocks and tiles that
+    """Preparation and sixteen-token recurrence of the hybrid layers' prompts (fewer rows than taps, chunks and tiles that
     end in between, widths past 128) against convolution, gates and the stepwise recurrence in FP32."""
     from uniserve_v1_b200.ops import gated_delta as GD
     T, B, C, rep = sum(lens), len(lens), 2 * Hk * Dk + Hv * Dv, Hv // Hk

@@ -1073,7 +1073,7 @@ int rule_impl(const RuleArgs& a, int B, cudaStream_t stream) {
 
 int prep_impl(const ChannelPrep& a, cudaStream_t stream) {
   US_REQUIRE(a.x && a.cq && a.ck && a.cv && a.A_log && a.dt_bias && a.q && a.k && a.v && a.g && a.beta && a.cu &&
-             a.slots && a.pos && a.B >= 1 && a.rows >= 1 && a.H >= 1 && a.Hk >= 1 && a.H % a.Hk == 0);
+             a.slots && (a.pos || a.window) && a.B >= 1 && a.rows >= 1 && a.H >= 1 && a.Hk >= 1 && a.H % a.Hk == 0);
   US_REQUIRE(a.K == 1 || a.conv);
   US_REQUIRE(!a.one_token || a.rows == a.B);
   if (a.K < 1 || a.K > kMaxTaps || a.D < 1 || a.D > kMaxDim || a.V < 1 || a.V > kMaxDim)
@@ -1151,9 +1151,8 @@ US_API int us_window_delta_prep(const void* x, long long ldx, int off_q, int off
                                 float* v, float* g, float* beta, const int* cu, const int* slots, int B, int rows, int H,
                                 int Hk, int D, int V, int K, int bf16, void* stream_) {
   US_REQUIRE(K >= 2);
-  // (positions are not read: the kernels' checks only ask for a table)
   ChannelPrep a{x, ldx, off_q, off_k, off_v, off_b, cq, ck, cv, nullptr, 0, off_a, A, dt_bias, conv,
-                q, k, v, g, beta, cu, slots, cu, B, rows, H, Hk, D, V, K, bf16, 0, 1};
+                q, k, v, g, beta, cu, slots, nullptr, B, rows, H, Hk, D, V, K, bf16, 0, 1};
   return prep_impl(a, (cudaStream_t)stream_);
 }
 

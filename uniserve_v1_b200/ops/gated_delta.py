@@ -115,8 +115,10 @@ def gated_delta_rule_packed(q, k, v, state, cu, slots, g=None, beta=None, raw=No
     return out
 
 
-# Rows per sequence from which the hybrid layers run the four-token recurrence behind one preparation launch; below,
-# its scratch and two more launches cost as much as the recurrence token by token (0.73 us a token and sequence).
+# Rows per sequence from which the hybrid layers run the sixteen-token recurrence behind one preparation launch.  Its
+# kernels are the slower ones up to 38 rows (32 heads of 128 x 128, by tokens / here: 8 rows 19 / 28 us, 16 24 / 34, 32 33 / 36,
+# 48 43 / 37, 128 93 / 49), its launches the faster ones for the host at any (84 / 65 us a layer, which is what a prompt of
+# up to 64 rows waits for: four layers of 16 rows 1197 / 1176 us, 64 1216 / 1185, 128 1575 / 1433).  Sixteen lies between.
 MIXER_MIN_ROWS = 16
 
 

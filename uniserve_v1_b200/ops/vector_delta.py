@@ -175,7 +175,8 @@ def vector_delta_rule(q, k, v, g, state, m: SeqMeta, beta=None, n=None, p=None):
         for t in (q, k, v, g, state):
             assert t.dtype == torch.float32 and t.is_contiguous()
         out = torch.empty(T, H, V, dtype=torch.float32, device=q.device)
-        if not general and few_tokens(T, max(m.lengths) if m.lengths else T, H, D, g.dim() == 3):
+        longest = 1 if m.one_token else max(m.lengths) if m.lengths else T
+        if not general and few_tokens(T, longest, H, D, g.dim() == 3):
             N.call("us_token_delta_rule", int(g.dim() == 3), N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(g), N.ptr(beta),
                    N.ptr(state), N.ptr(out), N.ptr(m.cu), N.ptr(m.slots), N.ptr(m.positions), m.slots.shape[0], H, Hk, D,
                    V, N.stream())
