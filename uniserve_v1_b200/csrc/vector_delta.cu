@@ -854,8 +854,12 @@ constexpr int kStepState = 64 * 1024;   // most bytes of a head's state: three C
 // two), and the vectors' loads do not queue behind it.  A thread multiplies every RG-th row x 4 columns; LQ threads
 // span the value columns.  Sums over key channels meet in shared memory.  64 sequences of 32 heads of 128 x 128 (268 MB, 41 us of
 // copying): 99 us with the state in registers, 79 here; what is left are the phases of a CTA, one after the other.
-template <int LQ, int RULE>
-__global__ void __launch_bounds__(kStepThreads, 3) vector_delta_step_kernel(const StepArgs a) {
+//
+// R > 0: a small state's rows, at most R of a thread, come straight into its registers, four CTAs to an SM (32 heads of
+// 64 x 64, a decay per head: 64 sequences 37 us through shared memory, 30 so; 256 162 and 123; 128 x 64, eight rows of a
+// thread: 67 in registers, 55 through shared memory).
+template <int LQ, int RULE, int R>
+__global__ void __launch_bounds__(kStepThreads, R > 0 ? 4 : 3) vector_delta_step_kernel(const StepArgs a) {
   US_PDL_PROLOGUE();
   constexpr bool GENERAL = RULE == kGeneral;
   constexpr int kVecs = RULE == kHead ? 2 : 3;        // vectors of D formed before v
@@ -876,7 +880,13 @@ __global__ void __launch_bounds__(kStepThreads, 3) vector_delta_step_kernel(cons
   extern __shared__ __align__(128) float held[];      // [D, V]
   __shared__ __align__(8) uint64_t arrived;
   const bool old = p0 > 0;                             // (a sequence's first token: zeros)
-  if (old && tid == 0) {
+  float4 S[R > 0 ? R : 1];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int row = rg + i * RG;
+    S[i] = old && on && row < D ? *reinterpret_cast<const float4*>(Sg + (long long)row * V) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (R == 0 && old && tid == 0) {
     tc::mbar_init(&arrived, 1);
     tc::mbar_fence_init();
     tc::mbar_expect_tx(&arrived, D * V * 4);
@@ -937,29 +947,39 @@ __global__ void __launch_bounds__(kStepThreads, 3) vector_delta_step_kernel(cons
       scal[4] = decay_exp(-expf(a.A_log[h]) * softplus_f(ld_any(a.x, xb + a.off_a + h, a.bf16) + a.bias[h]));
   }
   __syncthreads();
-  if (old && !tc::mbar_wait(&arrived, 0)) {
+  if (R == 0 && old && !tc::mbar_wait(&arrived, 0)) {
     us_dev_fail(a.status, US_DEV_TIMEOUT_FULL);
     tc::mbar_wait(&arrived, 0);                        // (nothing is left in flight when the CTA ends)
   }
   const float kinv = scal[1];
-  auto state = [&](int row) {                          // with the rule's decay
+  auto state = [&](int i, int row) {                   // with the rule's decay
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (old && on) x = *reinterpret_cast<const float4*>(held + row * V + cq4);
+    if (R > 0) x = S[i];
+    else if (old && on) x = *reinterpret_cast<const float4*>(held + row * V + cq4);
     if (!GENERAL) {
       const float g = RULE == kHead ? scal[4] : gs[row];
       x.x *= g; x.y *= g; x.z *= g; x.w *= g;
     }
     return x;
   };
+  auto each_row = [&](auto f) {
+    if (R > 0) {
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (rg + i * RG < D) f(i, rg + i * RG);
+    } else {
+#pragma unroll 4
+      for (int row = rg; row < D; row += RG) f(0, row);
+    }
+  };
   // ---- what the key sees ----
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-  for (int row = rg; row < D; row += RG) {
-    const float4 x = state(row);
+  each_row([&](int i, int row) {
+    const float4 x = state(i, row);
     const float k = ks[row] * kinv;
     acc.x = fmaf(x.x, k, acc.x); acc.y = fmaf(x.y, k, acc.y);
     acc.z = fmaf(x.z, k, acc.z); acc.w = fmaf(x.w, k, acc.w);
-  }
+  });
   auto gather = [&](float4 x) {                        // sum over the row groups
     *reinterpret_cast<float4*>(&red[rg][cq4]) = x;
     __syncthreads();
@@ -980,9 +1000,8 @@ __global__ void __launch_bounds__(kStepThreads, 3) vector_delta_step_kernel(cons
                     beta * (vv.w - seen.w));
   }
   acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-  for (int row = rg; row < D; row += RG) {
-    float4 x = state(row);
+  each_row([&](int i, int row) {
+    float4 x = state(i, row);
     if (GENERAL) {
       const float g = gs[row], k = ks[row], p = ps[row] * (k * kinv);
       x.x = fmaf(k, vv.x, fmaf(-p, u.x, g * x.x)); x.y = fmaf(k, vv.y, fmaf(-p, u.y, g * x.y));
@@ -996,7 +1015,7 @@ __global__ void __launch_bounds__(kStepThreads, 3) vector_delta_step_kernel(cons
     acc.x = fmaf(x.x, q, acc.x); acc.y = fmaf(x.y, q, acc.y);
     acc.z = fmaf(x.z, q, acc.z); acc.w = fmaf(x.w, q, acc.w);
     if (on) *reinterpret_cast<float4*>(Sg + (long long)row * V) = x;
-  }
+  });
   __syncthreads();                                     // the first sum has been read
   float4 o = gather(acc);
   const float qscale = GENERAL ? 1.f : scal[0] / sqrtf((float)D);
@@ -1023,9 +1042,13 @@ __global__ void __launch_bounds__(kStepThreads, 3) vector_delta_step_kernel(cons
 
 template <int LQ, int RULE>
 int launch_step(const StepArgs& a, int B, cudaStream_t stream) {
-  US_CUDA_CHECK((us::allow_shared<vector_delta_step_kernel<LQ, RULE>>(kStepState)));
-  US_CUDA_CHECK(us::launch_pdl(vector_delta_step_kernel<LQ, RULE>, dim3(a.H, B), dim3(kStepThreads),
-                               (size_t)a.D * a.V * sizeof(float), stream, a));
+  const dim3 grid(a.H, B), block(kStepThreads);
+  if (us::ceil_div(a.D, kStepThreads / LQ) <= 4) {
+    US_CUDA_CHECK(us::launch_pdl(vector_delta_step_kernel<LQ, RULE, 4>, grid, block, 0, stream, a));
+    return US_OK;
+  }
+  US_CUDA_CHECK((us::allow_shared<vector_delta_step_kernel<LQ, RULE, 0>>(kStepState)));
+  US_CUDA_CHECK(us::launch_pdl(vector_delta_step_kernel<LQ, RULE, 0>, grid, block, (size_t)a.D * a.V * sizeof(float), stream, a));
   return US_OK;
 }
 
