@@ -16,6 +16,7 @@ project paths.
 from __future__ import annotations
 
 import ctypes
+import gc
 from array import array
 from dataclasses import dataclass, field
 from typing import Optional
@@ -307,8 +308,16 @@ class CausalLmRunner:
             self._pool = torch.cuda.graph_pool_handle()
         before = N.launch_count
         self.announce(self._decode_kind("capture", B), B)
-        with torch.cuda.graph(graph, pool=self._pool):
-            logits, sampled = self._decode_body(blk, B, variant)
+        # The collector may not run meanwhile: a dead runner that it finds gives its graphs back, and that is not
+        # permitted during a capture and spoils it.
+        collects = gc.isenabled()
+        gc.disable()
+        try:
+            with torch.cuda.graph(graph, pool=self._pool):
+                logits, sampled = self._decode_body(blk, B, variant)
+        finally:
+            if collects:
+                gc.enable()
         launches = N.launch_count - before
         blk.dev.copy_(saved)
         torch.cuda.synchronize()
